@@ -450,42 +450,48 @@ void hgx_result_free(hgx_result* r) { delete r; }
 
 hgx_status hgx_engine_stage_times(hgx_engine* e, double* out, uint64_t* launches) {
     if (!e || !out) return fail(HGX_ERR_INVALID, "null argument");
-    const auto& t = e->engine.times();
-    out[0] = t.count;
-    out[1] = t.scan;
-    out[2] = t.expand;
-    out[3] = t.select;
-    out[4] = t.materialize;
-    out[5] = t.branchial;
-    out[6] = t.roots;
-    out[7] = t.count + t.scan + t.expand + t.expand_warp + t.select + t.materialize + t.branchial + t.roots;
-    if (launches) *launches = t.launches;
-    return HGX_OK;
+    return guarded([&] {
+        const auto& t = e->engine.times();
+        out[0] = t.count;
+        out[1] = t.scan;
+        out[2] = t.expand;
+        out[3] = t.select;
+        out[4] = t.materialize;
+        out[5] = t.branchial;
+        out[6] = t.roots;
+        out[7] = t.count + t.scan + t.expand + t.expand_warp + t.select + t.materialize + t.branchial + t.roots;
+        if (launches) *launches = t.launches;
+        return HGX_OK;
+    });
 }
 
 hgx_status hgx_engine_expand_stats(hgx_engine* e, uint64_t* out) {
     if (!e || !out) return fail(HGX_ERR_INVALID, "null argument");
-    const auto& t = e->engine.times();
-    out[0] = t.expand_bytes;
-    out[1] = t.expand_hbm_bytes;
-    out[2] = t.children;
-    out[3] = t.wl_rounds;
-    out[4] = t.expand_launches;
-    out[5] = t.warp_bytes;
-    out[6] = t.warp_hbm_bytes;
-    out[7] = t.warp_children;
-    out[8] = t.warp_rounds;
-    out[9] = static_cast<uint64_t>(t.expand_warp * 1e6);   // warp kernel time, ns
-    out[10] = t.walk_launches;
-    return HGX_OK;
+    return guarded([&] {
+        const auto& t = e->engine.times();
+        out[0] = t.expand_bytes;
+        out[1] = t.expand_hbm_bytes;
+        out[2] = t.children;
+        out[3] = t.wl_rounds;
+        out[4] = t.expand_launches;
+        out[5] = t.warp_bytes;
+        out[6] = t.warp_hbm_bytes;
+        out[7] = t.warp_children;
+        out[8] = t.warp_rounds;
+        out[9] = static_cast<uint64_t>(t.expand_warp * 1e6);   // warp kernel time, ns
+        out[10] = t.walk_launches;
+        return HGX_OK;
+    });
 }
 
 hgx_status hgx_engine_result_stats(hgx_engine* e, uint64_t* out) {
     if (!e || !out) return fail(HGX_ERR_INVALID, "null argument");
-    const auto& t = e->engine.times();
-    out[0] = t.result_streamed;
-    out[1] = t.result_chunks;
-    return HGX_OK;
+    return guarded([&] {
+        const auto& t = e->engine.times();
+        out[0] = t.result_streamed;
+        out[1] = t.result_chunks;
+        return HGX_OK;
+    });
 }
 
 hgx_status hgx_engine_stream(hgx_engine* e, void** stream) {

@@ -1410,6 +1410,66 @@ __device__ __forceinline__ uint64_t lane_wl(const Layout& L, char* sm, const Par
 // Kernels
 // ==========================================================================================
 
+// Admission of a batch of evolutions: its packed block (page-locked host memory, read over the bus)
+// scattered to the engine's arrays, and the fills that go with it, in one launch. Bound by the
+// bus's latency for a small batch (one round trip, all sections in flight); a section is read with
+// consecutive words per warp.
+struct AdmitArgs {
+    // the packed block's sections
+    const uint64_t* off;      // [n_roots] record offsets
+    const uint32_t *evos, *words, *ne, *nocc, *evo, *rules, *front;
+    // destinations of the appended runs
+    uint32_t *d_rules, *d_evos, *d_words, *d_front, *root_ids, *work;
+    uint32_t n_roots, n_words, n_rule_words, n_evos, n_front, evo0, s0, a0;
+    uint64_t edges0, edges1;  // initial edges (no producer)
+    uint64_t tab0, tab1;      // dedup table slots
+    uint64_t arena_words;     // the arena's top after this batch
+    uint32_t fresh;           // first admission of a run: clear the error flags and counters
+};
+
+__global__ void k_admit(DevPtrs P, AdmitArgs G) {
+    const uint64_t t = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x;
+    const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
+    for (uint64_t i = t; i < G.n_rule_words; i += stride) G.d_rules[i] = G.rules[i];
+    for (uint64_t i = t; i < uint64_t(G.n_evos) * (sizeof(DevEvo) / 4); i += stride) G.d_evos[i] = G.evos[i];
+    for (uint64_t i = t; i < G.n_words; i += stride) G.d_words[i] = G.words[i];
+    for (uint64_t i = t; i < G.n_front; i += stride) G.d_front[i] = G.front[i];
+    for (uint64_t i = t; i < G.n_roots; i += stride) {
+        const uint32_t s = G.s0 + static_cast<uint32_t>(i), a = G.a0 + static_cast<uint32_t>(i);
+        P.st_off[s] = G.off[i];
+        P.st_ne[s] = G.ne[i];
+        P.st_nocc[s] = G.nocc[i];
+        P.st_evo[s] = G.evo[i];
+        P.st_depth[s] = 0;
+        P.st_event[s] = a;
+        P.ev_in[a] = kNone;
+        P.ev_out[a] = s;
+        P.ev_kept[a] = 0;
+        P.state_of_arrival[a] = s;
+        G.root_ids[i] = s;
+    }
+    for (uint64_t i = G.edges0 + t; i < G.edges1; i += stride) P.edge_creator[i] = kNone;
+    for (uint64_t i = G.tab0 + t; i < G.tab1; i += stride) {
+        P.tab_keys[i] = 0ull;
+        P.tab_vals[i] = kNone;
+    }
+    for (uint64_t i = t; i < G.n_evos; i += stride) {
+        const uint64_t e = G.evo0 + i;
+        P.evo_classes[e] = 0;
+        P.evo_causal[e] = 0;
+        P.evo_states[e] = 0;
+        P.evo_sigs[e] = 0;
+        P.evo_cut[e] = kNone;
+        P.evo_stopped[e] = 0;
+    }
+    if (t < 8) G.work[t] = 0;
+    if (t == 0) *P.arena_top = G.arena_words;
+    if (G.fresh) {
+        if (t == 0) *P.err = 0;
+        if (t < 8) P.stats[t] = 0;
+    }
+}
+
 // Root states: hash the uploaded records and seed the dedup tables.
 __global__ void k_roots(DevPtrs P, const uint32_t* sids, uint32_t n, uint32_t* work, Layout L) {
     extern __shared__ __align__(16) char smem[];
@@ -1914,6 +1974,17 @@ __global__ void k_sync2_pack(const uint32_t* flag_rep, const uint32_t* flag_fron
         out[6] = static_cast<uint32_t>(states[0]);
         out[7] = static_cast<uint32_t>(states[0] >> 32);
         out[8] = stopped[0];
+    }
+}
+
+// The evolutions' counters of a counts-only run, straight into mapped page-locked memory.
+__global__ void k_counts_pack(DevPtrs P, uint32_t nevo, int sigs, unsigned long long* out) {
+    for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < nevo; e += gridDim.x * blockDim.x) {
+        out[e] = P.evo_causal[e];
+        out[nevo + e] = P.evo_classes[e];
+        out[2ull * nevo + e] = P.evo_states[e];
+        out[3ull * nevo + e] = P.evo_stopped[e];
+        out[4ull * nevo + e] = sigs ? P.evo_sigs[e] : 0ull;
     }
 }
 
@@ -3025,6 +3096,192 @@ __global__ void k_scan_down(ScanSet S, uint32_t n, const uint32_t* sums, uint32_
         ex += v[k];
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) out[n] = sm ? sm[nb] : total;
+}
+
+// ------------------------------------------------------------------------------------------
+// Small single-evolution results: chunk totals, emission, copy. Every block of the first two owns
+// one contiguous run of the events and one of the states; the emission takes its start offsets from
+// the totals of the blocks before it, so the three launches need no scan and no host round trip
+// between them. Latency-bound at these sizes: the work is launches and dependent loads, not bytes.
+// The copy writes 16 bytes a lane, whole 512-byte lines a warp, which the bus takes at its full rate
+// (the emission's own stores to host memory would be partial lines).
+// ------------------------------------------------------------------------------------------
+struct FinSmall {
+    uint32_t R, E, S, rule_begin;
+    uint64_t B;
+    uint32_t causal, edges, ids, sig;   // which arrays are wanted
+    uint32_t* sums;                     // [3][blocks] causal triples, state edges, occurrences
+    uint8_t* stage;                     // the arrays, in hgx_array order, 16-byte aligned
+    unsigned long long* bytes;          // staged bytes (device)
+    const uint32_t* pairs;
+    unsigned long long* head;           // page-locked: array counts, classes, stopped, signatures
+    uint8_t* host;                      // page-locked result block
+};
+
+// Element counts of the arrays from the totals, and their byte offsets.
+__device__ __forceinline__ void fin_small_layout(const FinSmall& F, uint32_t C, uint32_t K, uint32_t T,
+                                                     uint32_t V, uint64_t* count, uint64_t* off) {
+    const uint64_t c[kArr] = {F.S, F.S, 4ull * F.E, 3ull * K, 2 * F.B, F.E + 1ull, C, 2ull * F.E,
+                              F.edges ? F.S + 1ull : 1ull, F.ids ? T : 0u, F.edges ? T : 0u,
+                              F.edges ? F.S + 1ull : 1ull, F.edges ? V : 0u, F.sig ? F.E : 0u};
+    uint64_t at = 0;
+    for (uint32_t i = 0; i < kArr; ++i) {
+        const uint64_t eb = i == 10 ? 1u : (i == 0 || i == 13 ? 8u : 4u);
+        count[i] = c[i];
+        off[i] = at;
+        at += (c[i] * eb + 15) / 16 * 16;
+    }
+}
+
+__device__ __forceinline__ uint32_t causal_of(const DevPtrs& P, uint32_t e) {
+    const uint32_t co = P.ev_coff[e], k = P.rules[P.ev_rule[e]].n_lhs;
+    uint32_t c = 0;
+    for (uint32_t j = 0; j < k; ++j) c += P.ev_cprod[co + j] != kNone ? 1u : 0u;
+    return c;
+}
+
+__global__ void __launch_bounds__(256) k_fin_small_sums(DevPtrs P, FinSmall F) {
+    __shared__ uint32_t sh[3];
+    if (threadIdx.x < 3) sh[threadIdx.x] = 0;
+    __syncthreads();
+    const uint32_t G = gridDim.x, b = blockIdx.x;
+    const uint32_t ec = (F.E + G - 1) / G, sc = (F.S + G - 1) / G;
+    uint32_t k = 0, ne = 0, no = 0;
+    if (F.causal)
+        for (uint32_t i = b * ec + threadIdx.x; i < min(F.E, (b + 1) * ec); i += 256) k += causal_of(P, F.R + i);
+    if (F.edges)
+        for (uint32_t i = b * sc + threadIdx.x; i < min(F.S, (b + 1) * sc); i += 256) {
+            ne += P.st_ne[i];
+            no += P.st_nocc[i];
+        }
+    k = warp_sum32(k);
+    ne = warp_sum32(ne);
+    no = warp_sum32(no);
+    if (lane_id() == 0) {
+        atomicAdd(&sh[0], k);
+        atomicAdd(&sh[1], ne);
+        atomicAdd(&sh[2], no);
+    }
+    __syncthreads();
+    if (threadIdx.x < 3) F.sums[threadIdx.x * G + b] = sh[threadIdx.x];
+}
+
+__global__ void __launch_bounds__(256) k_fin_small_emit(DevPtrs P, FinSmall F) {
+    __shared__ uint32_t sh[33], pre[3], all[3];
+    __shared__ uint64_t off[kArr], count[kArr];
+    __shared__ uint32_t ebase[256], vbase[256];
+    const uint32_t G = gridDim.x, b = blockIdx.x, tid = threadIdx.x, lane = lane_id();
+    if (tid < 96) {   // warp a: array a's prefix before this block and its total
+        const uint32_t a = tid >> 5;
+        uint32_t p = 0, t = 0;
+        for (uint32_t i = lane; i < G; i += 32) {
+            const uint32_t x = F.sums[a * G + i];
+            t += x;
+            p += i < b ? x : 0u;
+        }
+        p = warp_sum32(p);
+        t = warp_sum32(t);
+        if (lane == 0) { pre[a] = p; all[a] = t; }
+    }
+    __syncthreads();
+    const uint32_t last = F.R + F.E - 1;
+    const uint32_t C = F.E ? P.ev_coff[last] + P.rules[P.ev_rule[last]].n_lhs : 0u;
+    if (tid == 0) {
+        fin_small_layout(F, C, all[0], all[1], all[2], count, off);
+        if (b == 0) {
+            for (uint32_t i = 0; i < kArr; ++i) F.head[i] = count[i];
+            F.head[kArr] = P.evo_classes[0];
+            F.head[kArr + 1] = P.evo_stopped[0];
+            F.head[kArr + 2] = F.sig ? P.evo_sigs[0] : 0ull;
+        }
+    }
+    __syncthreads();
+    auto arr = [&](uint32_t i) { return reinterpret_cast<uint32_t*>(F.stage + off[i]); };
+    // events
+    const uint32_t ec = (F.E + G - 1) / G, e1 = min(F.E, (b + 1) * ec);
+    uint32_t kbase = pre[0];
+    for (uint32_t i0 = b * ec; i0 < e1; i0 += 256) {
+        const uint32_t i = i0 + tid, e = F.R + i;
+        const bool live = i < e1;
+        const uint32_t kc = live && F.causal ? causal_of(P, e) : 0u;
+        uint32_t tot;
+        uint32_t w = kbase + block_excl_scan(kc, sh, tot);
+        kbase += tot;
+        if (!live) continue;
+        const uint32_t in = P.ev_in[e], r = P.ev_rule[e], co = P.ev_coff[e];
+        const DevRule& R = P.rules[r];
+        reinterpret_cast<uint4*>(arr(2))[i] = make_uint4(in, P.ev_out[e], r - F.rule_begin, P.st_depth[in] + 1);
+        arr(5)[i] = co;
+        reinterpret_cast<uint2*>(arr(7))[i] = make_uint2(P.ev_prod[e], R.n_rhs);
+        if (F.sig) reinterpret_cast<uint64_t*>(F.stage + off[13])[i] = P.ev_sig[e];
+        uint32_t* cons = arr(6);
+        uint32_t* tri = arr(3);
+        for (uint32_t j = 0; j < R.n_lhs; ++j) {
+            const uint32_t x = P.ev_cons[co + j];
+            cons[co + j] = x;
+            const uint32_t p = P.ev_cprod[co + j];
+            if (!F.causal || p == kNone) continue;
+            tri[3 * w] = p - F.R;
+            tri[3 * w + 1] = e - F.R;
+            tri[3 * w + 2] = x;
+            ++w;
+        }
+    }
+    if (b == 0 && tid == 0) arr(5)[F.E] = C;
+    // branchial pairs
+    for (uint64_t i = b * 256ull + tid; i < 2 * F.B; i += G * 256ull) arr(4)[i] = F.pairs[i] - F.R;
+    // states: hashes and depths, offsets and records (a warp per state over a tile of 256)
+    const uint32_t sc = (F.S + G - 1) / G, s1 = min(F.S, (b + 1) * sc);
+    uint32_t ep = pre[1], vp = pre[2];
+    for (uint32_t i0 = b * sc; i0 < s1; i0 += 256) {
+        const uint32_t i = i0 + tid;
+        const bool live = i < s1;
+        if (live) {
+            reinterpret_cast<uint64_t*>(F.stage + off[0])[i] = P.st_hash[i];
+            arr(1)[i] = P.st_depth[i];
+        }
+        if (!F.edges) continue;
+        uint32_t te, tv;
+        const uint32_t eo = ep + block_excl_scan(live ? P.st_ne[i] : 0u, sh, te);
+        const uint32_t vo = vp + block_excl_scan(live ? P.st_nocc[i] : 0u, sh, tv);
+        ep += te;
+        vp += tv;
+        if (live) {
+            arr(8)[i] = eo;
+            arr(11)[i] = vo;
+        }
+        ebase[tid] = eo;
+        vbase[tid] = vo;
+        __syncthreads();
+        const uint32_t n = min(256u, s1 - i0);
+        uint32_t* ids = arr(9);
+        uint8_t* ar = F.stage + off[10];
+        uint32_t* verts = arr(12);
+        for (uint32_t k = tid >> 5; k < n; k += 8) {
+            const uint32_t s = i0 + k, ne = P.st_ne[s], nocc = P.st_nocc[s], aw = (ne + 3) >> 2;
+            const uint32_t* rec = P.arena + P.st_off[s];
+            const uint32_t e0 = ebase[k], v0 = vbase[k];
+            for (uint32_t j = lane; j < ne; j += 32) {
+                if (F.ids) ids[e0 + j] = rec[j];
+                ar[e0 + j] = static_cast<uint8_t>(rec[ne + (j >> 2)] >> ((j & 3u) * 8u));
+            }
+            for (uint32_t j = lane; j < nocc; j += 32) verts[v0 + j] = rec[ne + aw + j];
+        }
+        __syncthreads();
+    }
+    if (b == 0 && tid == 0) {
+        arr(8)[F.edges ? F.S : 0] = F.edges ? all[1] : 0u;
+        arr(11)[F.edges ? F.S : 0] = F.edges ? all[2] : 0u;
+        *F.bytes = off[kArr - 1] + (count[kArr - 1] * 8 + 15) / 16 * 16;   // staged, for the copy
+    }
+}
+
+__global__ void __launch_bounds__(256) k_fin_small_copy(FinSmall F) {
+    const uint64_t n = *F.bytes / 16;
+    const uint4* s = reinterpret_cast<const uint4*>(F.stage);
+    uint4* d = reinterpret_cast<uint4*>(F.host);
+    for (uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; i < n; i += uint64_t(gridDim.x) * blockDim.x)
+        d[i] = s[i];
 }
 
 }  // namespace hgx
