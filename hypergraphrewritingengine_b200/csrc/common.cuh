@@ -135,6 +135,7 @@ enum ErrorBits : uint32_t {
     kErrArenaFull = 1u << 2,
     kErrBadRule = 1u << 3,
     kErrTrDepth = 1u << 4,       // transitive reduction past 64 levels
+    kErrBarrier = 1u << 6,       // a grid barrier's wait ran out
     kErrJoinCount = 1u << 5,     // a state's matches differ between the count and expand passes
 };
 

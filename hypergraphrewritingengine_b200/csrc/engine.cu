@@ -170,7 +170,7 @@ DevRule pack_rule(const RuleSpec& r) {
     return d;
 }
 
-uint32_t align_up(uint32_t x, uint32_t a) { return (x + a - 1) / a * a; }
+__host__ __device__ inline uint32_t align_up(uint32_t x, uint32_t a) { return (x + a - 1) / a * a; }
 
 // A streamed result's level is split into parts of at least this many frontier states.
 constexpr uint32_t kStreamPartStates = 16384;
@@ -184,12 +184,12 @@ enum class LayoutKind { Count, Lane, Warp };
 // per-vertex occurrence lists and a 32-match batch. Warp: plus the warp-per-child WL arrays.
 // NV: the most distinct vertices a staged state of this layout has (0 = bound them by NOCC); the
 // warp layout's per-vertex WL arrays and the vertex hash table are sized by it.
-Layout make_layout(uint32_t NE, uint32_t NOCC, const RuleMax& rm, LayoutKind kind, bool fwd = false,
-                   uint32_t mcap = kLaneJoinCap, bool index = false, uint32_t NV = 0) {
+__host__ __device__ Layout make_layout(uint32_t NE, uint32_t NOCC, const RuleMax& rm, LayoutKind kind,
+                                       bool fwd = false, uint32_t mcap = kLaneJoinCap,
+                                       bool index = false, uint32_t NV = 0) {
     const bool wl = kind == LayoutKind::Warp;
     const bool lane = kind == LayoutKind::Lane;
-    Layout L;
-    std::memset(&L, 0, sizeof(L));
+    Layout L{};
     NE = std::max<uint32_t>(NE, 1);
     NOCC = std::max<uint32_t>(NOCC, 1);
     L.NE = NE;
@@ -276,7 +276,7 @@ Layout make_layout(uint32_t NE, uint32_t NOCC, const RuleMax& rm, LayoutKind kin
         L.o_pconn = take(4, 4);
         L.o_pcnt = take(4 * kLaneVMax, 4);
         L.o_pdeg = take(2 * kLaneVMax, 2);
-        L.MCAP = std::max<uint32_t>(1, std::min<uint32_t>(mcap, kLaneJoinCap));
+        L.MCAP = std::max<uint32_t>(1, std::min<uint32_t>(mcap, +kLaneJoinCap));
         L.region_bytes = align_up(off, 16);   // batch and match list last: regions >= 1 stop here
         L.o_batch = take(32 * L.SB, 1);
         L.o_mlist = take(4 * L.MCAP, 4);
@@ -284,6 +284,8 @@ Layout make_layout(uint32_t NE, uint32_t NOCC, const RuleMax& rm, LayoutKind kin
     L.bytes = align_up(off, 16);
     return L;
 }
+
+#include "fused_levels.cuh"
 
 struct LaunchShape {
     uint32_t grid, block, smem;
@@ -447,6 +449,9 @@ struct Engine::Impl {
     DVec<unsigned long long> evo_new, ev_anc, ev_sig, evo_sigs;
     DVec<unsigned long long> ev_bmask;
     DVec<uint64_t> fin_rng;
+    DVec<FusedState> fused_state;   // grid-wide words of the small-level launch
+    DVec<uint32_t> fused_sums;
+    uint32_t fused_grid = 0;        // its blocks (one per SM); 0: cooperative launches unavailable
     DVec<uint32_t> fin_tab;   // many-evolution finalisation: bases, rule starts, boundary values
     DVec<uint64_t> fin_sec;   // many-evolution finalisation: section offsets
     // Per evolution: the contiguous id ranges it owns, one entry per level (roots first).
@@ -880,6 +885,18 @@ struct Engine::Impl {
                               (const void*)k_roots})
             HGX_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                 static_cast<int>(kMaxDynSmem)));
+        {
+            int coop = 0, sms = 0;
+            HGX_CUDA_CHECK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device));
+            HGX_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+            HGX_CUDA_CHECK(cudaFuncSetAttribute(k_levels, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                static_cast<int>(kFusedSmemMax)));
+            if (coop && occupancy(reinterpret_cast<const void*>(k_levels), kFusedThreads, kFusedSmemMax) >= 1)
+                fused_grid = std::min<uint32_t>(kNumSMs, static_cast<uint32_t>(sms));
+            fused_state.ensure(1, 0, st);
+            HGX_CUDA_CHECK(cudaMemsetAsync(fused_state.p, 0, sizeof(FusedState), st));
+            fused_sums.ensure(3 * kNumSMs, 0, st);
+        }
         arena_top.ensure(1, 0, st);
         err.ensure(1, 0, st);
         work.ensure(8, 0, st);
@@ -939,6 +956,9 @@ struct Engine::Impl {
         if (rb) cudaFreeHost(rb);
         if (h_sync) cudaFreeHost(h_sync);
         if (h_admit) cudaFreeHost(h_admit);
+        if (h_fused) cudaFreeHost(h_fused);
+        fused_state.release(st);
+        fused_sums.release(st);
         rules.release(st);
         evos.release(st);
         cudaStreamSynchronize(st);
@@ -1185,6 +1205,10 @@ struct Engine::Impl {
         std::vector<uint32_t> nes, noccs, h_evo, h_sid, h_front;
         std::vector<uint32_t> ids;
         uint64_t max_label = 0;
+        // dedup table slots per evolution: enough for its small levels without a rehash (32,768 for a
+        // single one, cleared in 2 us), a million slots over a batch, at least 256 each
+        uint64_t table_slots = 32768;
+        while (table_slots > 256 && table_slots * specs.size() > (1u << 20)) table_slots >>= 1;
         for (size_t i = 0; i < specs.size(); ++i) {
             const EvolutionSpec& spec = *specs[i];
             Packed& q = pk[i];
@@ -1235,7 +1259,7 @@ struct Engine::Impl {
             }
             words.insert(words.end(), q.words.begin(), q.words.end());
             // dedup table region
-            const uint64_t cap = next_pow2(std::max<uint64_t>(256, 4ull * nr));
+            const uint64_t cap = next_pow2(std::max<uint64_t>(table_slots, 4ull * nr));
             d.table_off = tab_slots;
             d.table_mask = cap - 1;
             tab_slots += cap + 1;
@@ -1901,6 +1925,188 @@ struct Engine::Impl {
     std::vector<uint64_t> sub_front;               // per evolution: next-frontier states so far
     std::vector<uint8_t> sub_part;                 // per evolution: in this level's frontier
 
+    // ---- small levels in one cooperative launch (fused_levels.cuh)
+    //
+    // Runs up to `most` levels of the frontier on the device and takes their records over. Returns
+    // the levels done; a level it leaves (too large, a cap within reach, a table to grow) is run by
+    // level(). Not used where a run needs what the launch does not do: match forwarding, per-stage
+    // timing, a device-memory ceiling (the launch reserves by bounds, which could pass a ceiling
+    // that the level's own sizes meet).
+    static constexpr size_t kFusedSmemMax = 200 * 1024;
+    uint32_t* h_fused = nullptr;
+    uint32_t* d_fused = nullptr;
+    size_t h_fused_words = 0;
+    uint32_t fused_levels(const RunOptions& opt, uint32_t most) {
+        if (!fused_grid || opt.forwarding || timing == 1 || budget.limit) return 0;
+        const size_t nevo = h_evos.size();
+        uint32_t done = 0;
+        bool grown = false;
+        while (done < most && frontier_size) {
+            if (uint64_t(frontier_size) * rm.stride > kFusedItems) break;
+            const uint32_t levels = std::min<uint32_t>({most - done, kFusedLevels,
+                                                        std::max<uint32_t>(1, static_cast<uint32_t>(4096 / nevo))});
+            const size_t words = kReportWords + kFusedLevels * kLevelWords + size_t(levels) * nevo * kRangeWords;
+            if (words > h_fused_words) {
+                HGX_CUDA_CHECK(cudaStreamSynchronize(st));
+                if (h_fused) HGX_CUDA_CHECK(cudaFreeHost(h_fused));
+                h_fused = nullptr;
+                h_fused_words = 0;
+                const size_t n = std::max<size_t>(words + words / 2, 4096);
+                HGX_CUDA_CHECK(cudaHostAlloc(reinterpret_cast<void**>(&h_fused), n * 4, cudaHostAllocMapped));
+                HGX_CUDA_CHECK(cudaHostGetDevicePointer(reinterpret_cast<void**>(&d_fused), h_fused, 0));
+                h_fused_words = n;
+            }
+            std::memset(h_fused, 0, words * 4);
+            if (opt.event_keys) fused_sig_tables();
+            counts.ensure(kFusedItems + 1, 0, st);
+            for (auto* v : {&item_ev, &item_cons, &item_prod, &item_fresh}) v->ensure(kFusedItems + 1, 0, st);
+            grow_events(n_events);
+            ev_bmask.ensure(n_events, n_events, st);
+            if (opt.transitive_reduction) ev_anc.ensure(n_events, n_events, st);
+            if (opt.event_keys) ev_sig.ensure(n_events, n_events, st);
+            FusedArgs G;
+            std::memset(&G, 0, sizeof(G));
+            G.fs = fused_state.p;
+            G.front[0] = frontier.p;
+            G.front[1] = next_frontier.p;
+            G.cnt = counts.p;
+            G.item_ev = item_ev.p;
+            G.item_cons = item_cons.p;
+            G.item_prod = item_prod.p;
+            G.item_fresh = item_fresh.p;
+            G.new_event = new_state_event.p;
+            G.sums = fused_sums.p;
+            G.bpairs = bpairs.p;
+            G.evo_last = evo_last_ev.p;
+            G.out = d_fused;
+            uint64_t re = std::min<uint64_t>({ev_in.cap, ev_rule.cap, ev_coff.cap, ev_prod.cap, ev_fresh.cap,
+                                              ev_out.cap, ev_kept.cap, ev_hash.cap, ev_nv.cap,
+                                              state_of_arrival.cap, ev_bmask.cap});
+            if (opt.transitive_reduction) re = std::min<uint64_t>(re, ev_anc.cap);
+            if (opt.event_keys) re = std::min<uint64_t>(re, ev_sig.cap);
+            G.room_events = re;
+            G.room_states = std::min<uint64_t>({st_off.cap, st_hash.cap, st_ne.cap, st_nocc.cap, st_evo.cap,
+                                                st_depth.cap, st_event.cap, st_ev0.cap, st_evn.cap, st_nv.cap});
+            G.room_cons = std::min<uint64_t>(ev_cons.cap, ev_cprod.cap);
+            G.room_edges = edge_creator.cap;
+            G.room_pairs = bpairs.cap / 2;
+            G.room_arena = arena.cap;
+            G.room_front = static_cast<uint32_t>(std::min<uint64_t>({frontier.cap, next_frontier.cap, new_state_event.cap, 0xFFFFFFFFull}));
+            G.arena_words = arena_words;
+            G.n_pairs = n_bpairs;
+            G.n_states = static_cast<uint32_t>(n_states);
+            G.n_events = static_cast<uint32_t>(n_events);
+            G.n_edges = static_cast<uint32_t>(n_edges);
+            G.n_cons = static_cast<uint32_t>(n_cons);
+            G.next_vertex = static_cast<uint32_t>(next_vertex);
+            G.F = frontier_size;
+            G.stride = rm.stride;
+            G.nevo = static_cast<uint32_t>(nevo);
+            G.levels = levels;
+            G.ne_bound = ne_bound;
+            G.no_bound = nocc_bound;
+            G.ev_keys = opt.event_keys;
+            G.tr = opt.transitive_reduction;
+            G.branchial = opt.branchial;
+            G.index = opt.join_index;
+            G.rm = rm;
+            // shared memory for a full block of warps a few levels on, within the launch's limit (a
+            // larger state has fewer warps a block, down to one)
+            const uint32_t ahead = std::min<uint32_t>(levels, 6);
+            const Layout Lw = make_layout(ne_bound + ahead * rm.grow_e, nocc_bound + ahead * rm.grow_o, rm,
+                                          LayoutKind::Warp, false, kLaneJoinCap, opt.join_index != 0);
+            G.smem = static_cast<uint32_t>(std::min<size_t>(std::max<size_t>(size_t(Lw.bytes) * kFusedWarps, 16 * 1024),
+                                                            kFusedSmemMax));
+            DevPtrs P = ptrs();
+            void* args[] = {&P, &G};
+            HGX_CUDA_CHECK(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_levels), dim3(fused_grid),
+                                                       dim3(kFusedThreads), args, G.smem, st));
+            check_launch();
+            sync_st();
+            const volatile uint32_t* o = h_fused;
+            const uint32_t stop = o[0], n = o[1];
+            if (o[3] & kErrTrDepth)
+                throw std::invalid_argument("transitive reduction supports evolutions of at most 64 levels");
+            if (o[3]) throw std::runtime_error("hgx: device error flags 0x" + std::to_string(o[3]));
+            if (sr.on && n) stream_issue();   // an earlier range's result chunk (its counts are here)
+            const uint64_t s_old = n_states, e_old = n_events, b_old = n_bpairs;
+            for (uint32_t lv = 0; lv < n; ++lv) {
+                const uint32_t* q0 = h_fused + kReportWords + kFusedLevels * kLevelWords + size_t(lv) * nevo * kRangeWords;
+                const uint32_t* rec = h_fused + kReportWords + lv * kLevelWords;
+                for (size_t e = 0; e < nevo; ++e) {
+                    const uint32_t* q = q0 + e * kRangeWords;
+                    if (!q[8] || evo_done[e]) continue;
+                    if (q[1] > q[0]) evo_ranges[e].events.emplace_back(q[0], q[1]);
+                    if (q[3] > q[2]) evo_ranges[e].states.emplace_back(q[2], q[3]);
+                    if (opt.branchial && q[5] > q[4]) evo_ranges[e].pairs.emplace_back(q[4], q[5]);
+                    if (q[7] == q[6]) {
+                        evo_done[e] = 1;
+                        finished.push_back(static_cast<uint32_t>(e));
+                    }
+                }
+                const uint64_t mne = rec[5], mno = rec[6];
+                n_events += rec[1];
+                n_states += rec[2];
+                n_bpairs += rec[4];
+                arena_words += rec[2] * (mne + (mne + 3) / 4 + mno);
+                ne_bound = static_cast<uint32_t>(mne);
+                nocc_bound = static_cast<uint32_t>(mno);
+                run_ne = std::max(run_ne, mne);
+                run_no = std::max(run_no, mno);
+                frontier_size = rec[3];
+                if (rec[1] && rec[2]) {
+                    hist.valid = true;
+                    hist.ev_per_state = double(rec[1]) / double(rec[0]);
+                    hist.ev_per_new = double(rec[1]) / double(rec[2]);
+                }
+            }
+            n_cons += o[14] | (uint64_t(o[15]) << 32);
+            n_edges += o[16];
+            next_vertex += o[17];
+            if (o[2]) std::swap(frontier, next_frontier);
+            hist.have_ok = nevo == 1;
+            hist.have[0] = o[4] | (uint64_t(o[5]) << 32);
+            hist.have[1] = o[6] | (uint64_t(o[7]) << 32);
+            hist.stopped = o[8];
+            done += n;
+            if (n) grown = false;
+            if (sr.on && n) {
+                const uint32_t q[7] = {uint32_t(e_old), uint32_t(n_events), uint32_t(s_old), uint32_t(n_states),
+                                       uint32_t(b_old), uint32_t(n_bpairs), 0};
+                stream_prep(q, run_ne, run_no);
+            }
+            if (stop == kStopDone) continue;
+            if (stop != kStopRoom || grown) break;
+            // room for the level it stopped at, then again
+            grown = true;
+            grow_events(n_events + o[9]);
+            grow_states(n_states + o[9]);
+            ev_bmask.ensure(n_events + o[9], n_events, st);
+            if (opt.transitive_reduction) ev_anc.ensure(n_events + o[9], n_events, st);
+            if (opt.event_keys) ev_sig.ensure(n_events + o[9], n_events, st);
+            ev_cons.ensure(n_cons + o[10], n_cons, st);
+            ev_cprod.ensure(n_cons + o[10], n_cons, st);
+            edge_creator.ensure(n_edges + o[11], n_edges, st);
+            if (opt.branchial) bpairs.ensure(2ull * (n_bpairs + o[12]), 2ull * n_bpairs, st);
+            arena.ensure(arena_words + o[13], arena_words, st);
+            frontier.ensure(std::max<uint64_t>(o[9], frontier_size), frontier_size, st);
+            next_frontier.ensure(o[9], 0, st);
+            new_state_event.ensure(o[9], 0, st);
+        }
+        return done;
+    }
+    // Signature tables for the evolutions still running that have none yet.
+    void fused_sig_tables() {
+        size_t lo = h_evos.size(), hi = 0;
+        for (size_t e = 0; e < h_evos.size(); ++e) {
+            if (evo_done[e] || h_evos[e].sig_mask) continue;
+            regrow_region(h_evos[e].sig_off, h_evos[e].sig_mask, (h_evos[e].table_mask + 1) / 2);
+            lo = std::min(lo, e);
+            hi = e + 1;
+        }
+        upload_evos(lo, hi);
+    }
+
     bool level(const RunOptions& opt) {
         const uint32_t F = frontier_size;
         if (F == 0) return false;
@@ -2508,7 +2714,10 @@ std::vector<EvolutionResult> Engine::run(const std::vector<EvolutionSpec>& specs
     for (const auto& s : specs) ptrs.push_back(&s);
     const std::vector<uint32_t> ids = I.admit_many(ptrs);
     I.stream_begin(opt);
-    while (I.level(opt)) {}
+    while (I.frontier_size) {
+        I.fused_levels(opt, UINT32_MAX);   // as many small levels as it takes
+        if (I.frontier_size) I.level(opt);
+    }
     std::vector<EvolutionResult> out;
     if (!opt.readback) {
         I.read_counts(ids, out, opt.event_keys != 0);
@@ -2545,7 +2754,8 @@ std::vector<uint32_t> Engine::admit(const std::vector<EvolutionSpec>& specs) {
 }
 bool Engine::step(const RunOptions& opt) {
     BudgetScope scope(&impl_->budget);
-    return impl_->level(opt);
+    if (!impl_->fused_levels(opt, 1)) return impl_->level(opt);
+    return impl_->frontier_size > 0;
 }
 void Engine::set_device_limit(uint64_t bytes) { impl_->budget.limit = bytes; }
 uint64_t Engine::device_limit() const { return impl_->budget.limit; }

@@ -1848,39 +1848,38 @@ __global__ void k_cprod(DevPtrs P, uint32_t ev_base, uint32_t n) {
 // of the stored (producer, consumer) relation that the reference computes
 // (common/include/hgcommon/transitive_reduction.hpp:36-94; kept triples: those whose pair
 // survives, hypergraph/include/hypergraph/causal_graph.hpp:295-305).
-__global__ void k_tr(DevPtrs P, uint32_t ev_base, uint32_t n) {
-    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-        const uint32_t e = ev_base + t;
-        const uint32_t co = P.ev_coff[e], k = P.rules[P.ev_rule[e]].n_lhs;
-        uint32_t q[kMaxPatternEdges];
-        uint32_t lv[kMaxPatternEdges];
-        unsigned long long qa[kMaxPatternEdges];
-        unsigned long long anc = 0;
-        bool deep = false;
-        for (uint32_t i = 0; i < k; ++i) {
-            q[i] = P.ev_cprod[co + i];
-            lv[i] = 0;
-            qa[i] = 0;
-            if (q[i] == kNone) continue;
-            lv[i] = P.st_depth[P.ev_in[q[i]]];
-            deep |= lv[i] >= 64;
-            qa[i] = P.ev_anc[q[i]];
-            anc |= qa[i] | (1ull << (lv[i] & 63u));
-        }
-        P.ev_anc[e] = anc;
-        if (deep) { atomicOr(P.err, kErrTrDepth); continue; }
-        for (uint32_t i = 0; i < k; ++i) {
-            if (q[i] == kNone) continue;
-            bool implied = false;
-            for (uint32_t j = 0; j < k && !implied; ++j)
-                implied = q[j] != kNone && q[j] != q[i] && ((qa[j] >> lv[i]) & 1ull);
-            if (implied) P.ev_cprod[co + i] = kNone;
-        }
+__device__ __forceinline__ void reduce_event(const DevPtrs& P, uint32_t e) {
+    const uint32_t co = P.ev_coff[e], k = P.rules[P.ev_rule[e]].n_lhs;
+    uint32_t q[kMaxPatternEdges];
+    uint32_t lv[kMaxPatternEdges];
+    unsigned long long qa[kMaxPatternEdges];
+    unsigned long long anc = 0;
+    bool deep = false;
+    for (uint32_t i = 0; i < k; ++i) {
+        q[i] = P.ev_cprod[co + i];
+        lv[i] = 0;
+        qa[i] = 0;
+        if (q[i] == kNone) continue;
+        lv[i] = P.st_depth[P.ev_in[q[i]]];
+        deep |= lv[i] >= 64;
+        qa[i] = P.ev_anc[q[i]];
+        anc |= qa[i] | (1ull << (lv[i] & 63u));
+    }
+    P.ev_anc[e] = anc;
+    if (deep) { atomicOr(P.err, kErrTrDepth); return; }
+    for (uint32_t i = 0; i < k; ++i) {
+        if (q[i] == kNone) continue;
+        bool implied = false;
+        for (uint32_t j = 0; j < k && !implied; ++j)
+            implied = q[j] != kNone && q[j] != q[i] && ((qa[j] >> lv[i]) & 1ull);
+        if (implied) P.ev_cprod[co + i] = kNone;
     }
 }
 
-
-
+__global__ void k_tr(DevPtrs P, uint32_t ev_base, uint32_t n) {
+    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x)
+        reduce_event(P, ev_base + t);
+}
 
 // Per frontier state: its first event and first-rule event count (the record match forwarding
 // reads at the next level). Per evolution: first / one-past-last event of this level (the
@@ -2663,33 +2662,33 @@ __device__ __forceinline__ uint32_t seg_incl_scan(uint32_t x) {
 }
 
 // Write the edge record of every new state: parent edges minus consumed, then produced.
-// Groups of 32 new states per warp share one arena reservation and one level-maximum update;
+// Groups of 32 new states per warp share one arena reservation;
 // the group's states are then written 32 / S at a time, one per segment of S lanes (lanes =
 // parent edges), S chosen on the host from the level's largest parent (8, 16 or 32 edges per
 // pass), so a small parent does not leave most of the warp idle.
-// Held to 64 registers (4 blocks per SM; no spills): C2 materialise 0.99 -> 0.87 ms.
+// New states [j0, j1) of a level whose first is state_base, dealt in groups of 32 to warp w0 of
+// n_warps; scratch: the warp's (kMaxVars + kMaxPatternEdges) * 32 / S words of shared memory.
 template <uint32_t S>
-__global__ void __launch_bounds__(256, 4) k_materialize(DevPtrs P, LevelArgs A, uint32_t n_new) {
+__device__ __forceinline__ void materialize_states(const DevPtrs& P, const uint32_t* new_state_event,
+                                                   uint32_t state_base, uint32_t j0, uint32_t j1,
+                                                   uint32_t w0, uint32_t n_warps, uint32_t* scratch) {
     constexpr uint32_t G = 32 / S;
-    __shared__ uint32_t bind_sm[8][G][kMaxVars];
-    __shared__ uint32_t cons_sm[8][G][kMaxPatternEdges];
     const uint32_t lane = lane_id();
-    const uint32_t w = threadIdx.x >> 5;
     const uint32_t seg = lane / S, sl = lane & (S - 1);
     const uint32_t segbits = S == 32 ? 0xFFFFFFFFu : ((1u << S) - 1u);
-    uint32_t* bind = bind_sm[w][seg];
-    uint32_t* cons = cons_sm[w][seg];
+    uint32_t* bind = scratch + seg * (kMaxVars + kMaxPatternEdges);
+    uint32_t* cons = bind + kMaxVars;
+    const uint32_t n_new = j1;
     // groups of 32 new states per warp: record sizes by lane, one arena reservation per group
-    for (uint32_t g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; g * 32ull < n_new;
-         g += (gridDim.x * blockDim.x) >> 5) {
-        const uint32_t jl = g * 32 + lane;
-        uint32_t words = 0, gne = 0, gnocc = 0;
+    for (uint32_t g = w0; j0 + g * 32ull < n_new; g += n_warps) {
+        const uint32_t jl = j0 + g * 32 + lane;
+        uint32_t words = 0;
         // lane k loads state k's event, parent and rule once; the loop below takes them by
         // shuffle instead of repeating the chain of dependent loads per state
         uint32_t e_l = 0, f_l = 0, r_l = 0, pne_l = 0, pnocc_l = 0, coff_l = 0, pid_l = 0, fid_l = 0;
         unsigned long long poff_l = 0;
         if (jl < n_new) {
-            e_l = A.new_state_event[jl];
+            e_l = new_state_event[jl];
             f_l = P.ev_in[e_l];
             r_l = P.ev_rule[e_l];
             coff_l = P.ev_coff[e_l];
@@ -2699,35 +2698,29 @@ __global__ void __launch_bounds__(256, 4) k_materialize(DevPtrs P, LevelArgs A, 
             pne_l = P.st_ne[f_l];
             pnocc_l = P.st_nocc[f_l];
             poff_l = P.st_off[f_l];
-            gne = pne_l - R.n_lhs + R.n_rhs;
-            gnocc = pnocc_l - R.lhs_total + R.rhs_total;
+            const uint32_t gne = pne_l - R.n_lhs + R.n_rhs;
+            const uint32_t gnocc = pnocc_l - R.lhs_total + R.rhs_total;
             words = gne + ((gne + 3) >> 2) + gnocc;
-            P.st_nv[A.state_base + jl] = P.ev_nv[e_l];
+            P.st_nv[state_base + jl] = P.ev_nv[e_l];
         }
         const uint32_t inc = warp_incl_scan(words);
         const uint32_t total = __shfl_sync(0xFFFFFFFFu, inc, 31);
-        gne = warp_max32(gne);
-        gnocc = warp_max32(gnocc);
         unsigned long long base = 0;
-        if (lane == 0) {
-            base = atomicAdd(P.arena_top, static_cast<unsigned long long>(total));
-            atomicMax(&A.level_max[0], gne);
-            atomicMax(&A.level_max[1], gnocc);
-        }
+        if (lane == 0) base = atomicAdd(P.arena_top, static_cast<unsigned long long>(total));
         base = __shfl_sync(0xFFFFFFFFu, base, 0);
         if (base + total > P.arena_cap) {
             if (lane == 0) atomicOr(P.err, kErrArenaFull);
             continue;
         }
         const unsigned long long my_off = base + inc - words;
-        const uint32_t cnt = min(32u, n_new - g * 32);
+        const uint32_t cnt = min(32u, n_new - j0 - g * 32);
         for (uint32_t k0 = 0; k0 < cnt; k0 += G) {
             const uint32_t k = k0 + seg;               // this segment's state in the group
             const bool act = k < cnt;
             const uint32_t src = act ? k : 0u;
-            const uint32_t j = g * 32 + k;
+            const uint32_t j = j0 + g * 32 + k;
             const unsigned long long off = __shfl_sync(0xFFFFFFFFu, my_off, src);
-            const uint32_t sid = A.state_base + j;
+            const uint32_t sid = state_base + j;
             const DevRule& R = P.rules[__shfl_sync(0xFFFFFFFFu, r_l, src)];
             // every lane takes part in every shuffle (a full-mask shuffle that some lanes skip
             // never completes); inactive segments then zero what they took
@@ -2804,6 +2797,15 @@ __global__ void __launch_bounds__(256, 4) k_materialize(DevPtrs P, LevelArgs A, 
             __syncwarp();
         }
     }
+}
+
+// Held to 64 registers (4 blocks per SM; no spills): C2 materialise 0.99 -> 0.87 ms.
+template <uint32_t S>
+__global__ void __launch_bounds__(256, 4) k_materialize(DevPtrs P, LevelArgs A, uint32_t n_new) {
+    __shared__ uint32_t scratch[8][(kMaxVars + kMaxPatternEdges) * (32 / S)];
+    materialize_states<S>(P, A.new_state_event, A.state_base, 0, n_new,
+                          (blockIdx.x * blockDim.x + threadIdx.x) >> 5, (gridDim.x * blockDim.x) >> 5,
+                          scratch[threadIdx.x >> 5]);
 }
 
 // Branchial pairs (CausalGraph::record_branchial_overlaps, hypergraph/src/causal_graph.cpp:324-350):

@@ -1,0 +1,109 @@
+"""Small levels in one cooperative launch against the ordinary level pipeline.
+
+Per-stage timing (HGX_OPT_TIMING = 1) turns the launch off, so the same call runs on both paths;
+every result array must be equal, ids and order included. The cases sit at the edges of the
+launch's rule: levels just below and above its event limit, states around 63 / 64 edges (branchial
+masks, lane walk against warp join) and 96 (join index), several rules and roots, unary and mixed
+arities, a deleting rule, caps out of and within reach, evolutions that stop in different levels of
+one batch, and levels run one per call by the serving steps.
+"""
+import numpy as np
+import pytest
+
+import cases
+from hypergraphrewritingengine_b200 import Engine, api
+from hypergraphrewritingengine_b200 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+ARRAYS = ("state_hash", "state_depth", "events", "causal", "branchial", "event_cons_off",
+          "event_cons", "event_prod", "state_edge_off", "state_edge_ids", "state_arity",
+          "state_vert_off", "state_verts", "event_signature")
+
+
+def same_arrays(a, b, what):
+    for name in ARRAYS:
+        assert np.array_equal(getattr(a, name), getattr(b, name)), (what, name)
+    assert (a.num_classes, a.num_canonical_events, a.truncated) == \
+        (b.num_classes, b.num_canonical_events, b.truncated), what
+
+
+@pytest.fixture(scope="module")
+def engines():
+    both = Engine(0), Engine(0)
+    both[1].set_option(api.OPT_TIMING, 1)
+    yield both
+    for e in both:
+        e.close()
+
+
+def _chain(n):
+    return [[i, i + 1] for i in range(1, n)] + [[n, 1]]
+
+
+GROW = [([[0, 1], [1, 2]], [[0, 1], [1, 2], [2, 0]])]
+SINGLE = {name: (rules, roots, steps, False, 0) for name, rules, roots, steps in cases.all_full_cases()
+          if name.startswith("edge-") or name.startswith("corpus-")}
+SINGLE.update({
+    "wpp-7": ([cases.C2_RULE], [cases.C2_INIT], 7, True, 0),            # past the event limit
+    "wpp-full-4": ([cases.C2_RULE], [cases.C2_INIT], 4, False, 0),
+    "ternary-5": ([cases.C3_RULE], [cases.C3_INIT], 5, True, 0),
+    "cap-far": ([cases.C2_RULE], [cases.C2_INIT], 5, True, 100000),
+    "cap-near": ([cases.C2_RULE], [cases.C2_INIT], 6, True, 700),
+    "cap-full": ([cases.C1_RULE], [cases.C1_INIT], 5, False, 900),
+    "edges-62": (GROW, [_chain(62)], 2, True, 0),
+    "edges-63": (GROW, [_chain(63)], 2, True, 0),
+    "edges-64": (GROW, [_chain(64)], 2, True, 0),
+    "edges-97": (GROW, [_chain(97)], 2, True, 0),
+    "edges-97-roots": (GROW, [_chain(97), _chain(40), _chain(97)], 1, True, 0),
+    "no-match": ([([[0, 1, 2]], [[0, 1]])], [_chain(3)], 3, True, 0),
+    "long-lhs": ([([[0, 1], [1, 2], [2, 3], [3, 4], [4, 5]], [[0, 5], [5, 6]])], [_chain(12)], 3, True, 0),
+    "20-levels": ([([[0, 1]], [[1, 0]])], [_chain(5)], 20, True, 0),    # more levels than one launch takes
+})
+
+
+@pytest.mark.parametrize("reduce,keys", [(False, 0), (True, 3)])
+@pytest.mark.parametrize("name", sorted(SINGLE))
+def test_single_evolutions(engines, name, reduce, keys):
+    rules, roots, steps, quotient, cap = SINGLE[name]
+    out = []
+    for eng in engines:
+        eng.set_option(api.OPT_TRANSITIVE_REDUCTION, reduce)
+        eng.set_option(api.OPT_EVENT_SIGNATURE_KEYS, keys)
+        out.append(eng.evolve(rules, roots, steps, quotient=quotient, max_states=cap))
+        eng.set_option(api.OPT_TRANSITIVE_REDUCTION, False)
+        eng.set_option(api.OPT_EVENT_SIGNATURE_KEYS, 0)
+    same_arrays(*out, name)
+
+
+@pytest.mark.parametrize("n,cap", [(1, 50), (37, 200), (300, 4096)])
+def test_batches(engines, n, cap):
+    evs = [W.random_evolution(i, seed=71 + n, max_states=cap, edges_hi=40, steps_lo=0, steps_hi=4)
+           for i in range(n)]
+    for i, (a, b) in enumerate(zip(*(eng.evolve_batch(evs) for eng in engines))):
+        same_arrays(a, b, i)
+
+
+def test_record_options_and_serving_steps(engines):
+    evs = [W.random_evolution(i, seed=5, max_states=300, edges_hi=30, steps_hi=5) for i in range(12)]
+    for causal, branchial in ((False, True), (True, False)):
+        out = []
+        for eng in engines:
+            eng.set_option(api.OPT_RECORD_CAUSAL, causal)
+            eng.set_option(api.OPT_RECORD_BRANCHIAL, branchial)
+            eng.serve_reset()
+            jobs, keep = eng.make_jobs(evs)
+            ids = eng.serve_admit_batch(jobs, 7)
+            got, more = {}, 7
+            while len(got) < len(evs):
+                for k, r in zip(*(lambda d: (d, eng.serve_collect_batch(d)))(eng.serve_take_finished())):
+                    got[k] = r
+                if more < len(evs):     # one more request between the levels of the others
+                    ids.append(eng.serve_admit(jobs[more]))
+                    more += 1
+                eng.serve_step()
+            out.append([got[i] for i in ids])
+            eng.set_option(api.OPT_RECORD_CAUSAL, True)
+            eng.set_option(api.OPT_RECORD_BRANCHIAL, True)
+        for i, (a, b) in enumerate(zip(*out)):
+            same_arrays(a, b, (causal, branchial, i))
