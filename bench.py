@@ -297,7 +297,7 @@ def main():
     ap.add_argument("--no-extras", action="store_true", help="skip the batched comparison")
     ap.add_argument("--levels", type=int, default=8)
     ap.add_argument("--lane-join", type=int, default=0, choices=[0, 1, 2],
-                    help="small-state join: 0 autotuned (default), 1 warp join, 2 lane walk")
+                    help="small-state join: 0 default (lane walk), 1 warp join, 2 lane walk")
     ap.add_argument("--profile-run", action="store_true",
                     help="run the workload once, device-resident, and exit (for profilers)")
     ap.add_argument("--profile-workload", default="c2", choices=["c2", "c4", "large"],

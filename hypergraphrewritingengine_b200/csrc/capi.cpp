@@ -240,7 +240,7 @@ hgx_status hgx_engine_set_option(hgx_engine* e, hgx_option opt, uint64_t value) 
             e->opt.stream_result = static_cast<uint32_t>(value);
             return HGX_OK;
         case HGX_OPT_LANE_JOIN:
-            if (value > 2) return fail(HGX_ERR_INVALID, "lane join must be 0 (autotuned), 1 or 2");
+            if (value > 2) return fail(HGX_ERR_INVALID, "lane join must be 0 (default), 1 or 2");
             e->opt.lane_join = static_cast<uint32_t>(value);
             return HGX_OK;
         case HGX_OPT_EVENT_SIGNATURE_KEYS:

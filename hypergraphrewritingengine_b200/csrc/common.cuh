@@ -44,6 +44,7 @@ constexpr int kLaneVMax = 32;
 constexpr int kLaneVMaxSmall = 12;
 constexpr uint32_t kLaneFullStates = 148 * 4 * 8;
 constexpr int kLaneEMax = 64;
+constexpr uint32_t kSegEMax = 64;   // segment path (seg_wl.cuh): edges of a child
 constexpr int kLaneNMax = 64;    // neighbour entries a lane sorts for one vertex
 
 // Match forwarding: at most this many delta matches per state (else the state is re-joined), and

@@ -174,11 +174,13 @@ __host__ __device__ inline uint32_t align_up(uint32_t x, uint32_t a) { return (x
 
 // A streamed result's level is split into parts of at least this many frontier states.
 constexpr uint32_t kStreamPartStates = 16384;
+// Smallest level (children) of small binary states that the lane kernel takes from the segment one.
+constexpr uint32_t kLaneLevel = 1u << 20;
 // Results streamed only when the last one was at least this large (a small result's copy is
 // shorter than the per-range work streaming adds).
 constexpr uint64_t kStreamMinBytes = 64ull << 20;
 
-enum class LayoutKind { Count, Lane, Warp };
+enum class LayoutKind { Count, Lane, Warp, Seg };
 
 // Shared-memory carve-up per warp. Count: the parent and the join. Lane: plus the parent's
 // per-vertex occurrence lists and a 32-match batch. Warp: plus the warp-per-child WL arrays.
@@ -186,9 +188,9 @@ enum class LayoutKind { Count, Lane, Warp };
 // warp layout's per-vertex WL arrays and the vertex hash table are sized by it.
 __host__ __device__ Layout make_layout(uint32_t NE, uint32_t NOCC, const RuleMax& rm, LayoutKind kind,
                                        bool fwd = false, uint32_t mcap = kLaneJoinCap,
-                                       bool index = false, uint32_t NV = 0) {
+                                       bool index = false, uint32_t NV = 0, uint32_t seg = 32) {
     const bool wl = kind == LayoutKind::Warp;
-    const bool lane = kind == LayoutKind::Lane;
+    const bool lane = kind == LayoutKind::Lane || kind == LayoutKind::Seg;
     Layout L{};
     NE = std::max<uint32_t>(NE, 1);
     NOCC = std::max<uint32_t>(NOCC, 1);
@@ -252,6 +254,8 @@ __host__ __device__ Layout make_layout(uint32_t NE, uint32_t NOCC, const RuleMax
         L.o_vtab = take(4 * L.VT, 4);
         L.o_vtid = take(2 * L.VT, 2);
     }
+    L.VM = std::min<uint32_t>(L.NV, kind == LayoutKind::Lane || kind == LayoutKind::Seg ? kLaneVMax : 64);
+    L.o_vm = take(8 * L.VM, 8);
     if (index && !lane && NE > kJoinIndexMin) {
         L.XI = 1;
         L.o_xready = take(4, 4);
@@ -266,7 +270,19 @@ __host__ __device__ Layout make_layout(uint32_t NE, uint32_t NOCC, const RuleMax
         while (n2 < 2 * L.V) n2 <<= 1;
         L.o_srt = take(8 * (n2 + 1), 8);
     }
-    if (lane) {
+    if (kind == LayoutKind::Seg) {
+        L.o_ppk = take(4 * NE, 4);
+        L.RHS = rm.rhs;
+        L.SB = align_up(8 + 4 * rm.rhs + rm.lhs, 8);
+        L.MCAP = mcap;
+        L.SEGE = NE + rm.grow_e;
+        L.SEGN = L.SEGE * rm.arity * (rm.arity - 1);
+        L.SEGB = seg_scratch_bytes(seg, L.SEGE, L.SEGN);
+        L.o_batch = take(32 * L.SB, 16);
+        L.o_mlist = take(4 * L.MCAP, 4);
+        L.SEGB = align_up(L.SEGB, 8);
+        L.o_seg = take((32 / seg) * L.SEGB, 8);
+    } else if (lane) {
         L.SB = rm.lhs + rm.rhs_total;
         L.o_poff = take(2 * (kLaneVMax + 1), 2);
         L.o_pocc = take(2 * NOCC, 2);
@@ -410,17 +426,6 @@ struct Engine::Impl {
     cudaStream_t st = nullptr;
     int timing = 0;   // 0 off, 1 every stage, 2 the expand kernel only
     StageTimes times;
-    cudaEvent_t ev_a = nullptr, ev_b = nullptr;   // the join autotuner's measurement window
-    // Join autotuner for the lane expand kernel: per bucket b = floor(log2(children per frontier
-    // state)) and variant (0 warp join, 1 lane walk), the device time per child of large levels
-    // (exponential average). Each variant is tried once in the bucket; then the faster one runs
-    // (and keeps being measured). Small levels use the measured default (walk from 32
-    // children/state).
-    struct JoinTuner {
-        double ns[8][2] = {};
-        uint32_t n[8][2] = {};
-    } tuner;
-    static constexpr uint64_t kTuneMinChildren = 65536;
 
     // device arrays
     DVec<DevRule> rules;
@@ -445,7 +450,7 @@ struct Engine::Impl {
     DVec<uint32_t> bcount, boff, bpairs, scan_sums, sync_buf, root_ids;
     DVec<unsigned long long> stats, totals;
     DVec<uint8_t> fmode, fin;
-    DVec<uint32_t> fin_cnt, evo_frange, fin_ids, map_s, map_e, frng, slice_off;
+    DVec<uint32_t> fin_cnt, evo_frange, fin_ids, map_s, map_e, frng, slice_off, seg_off;
     DVec<unsigned long long> evo_new, ev_anc, ev_sig, evo_sigs;
     DVec<unsigned long long> ev_bmask;
     DVec<uint64_t> fin_rng;
@@ -855,6 +860,7 @@ struct Engine::Impl {
     uint64_t next_vertex = 0, arena_words = 0, tab_slots = 0;
     uint32_t frontier_size = 0;
     uint32_t ne_bound = 1, nocc_bound = 1;
+    bool uniform = true;      // each evolution's roots and right-hand sides share one arity, 2 or 3
     uint64_t run_ne = 1, run_no = 1;   // the run's largest state record so far (edges, occurrences)
     uint64_t launches = 0;
 
@@ -865,8 +871,6 @@ struct Engine::Impl {
         HGX_CUDA_CHECK(cudaSetDevice(device));
         HGX_CUDA_CHECK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
         HGX_CUDA_CHECK(cudaStreamCreateWithFlags(&cst, cudaStreamNonBlocking));
-        HGX_CUDA_CHECK(cudaEventCreate(&ev_a));
-        HGX_CUDA_CHECK(cudaEventCreate(&ev_b));
         HGX_CUDA_CHECK(cudaEventCreateWithFlags(&sr.ready, cudaEventDisableTiming));
         HGX_CUDA_CHECK(cudaMallocHost(reinterpret_cast<void**>(&sr.hsz), 4 * sizeof(uint32_t)));
         cudaMemPool_t pool;
@@ -880,6 +884,10 @@ struct Engine::Impl {
                               (const void*)k_expand_lanes2<true, kLaneRegions, false>})
             HGX_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                 static_cast<int>(kMaxDynSmem - 8192)));
+        for (const void* k : {(const void*)k_expand_seg<16, true>, (const void*)k_expand_seg<16, false>,
+                              (const void*)k_expand_seg<32, true>, (const void*)k_expand_seg<32, false>})
+            HGX_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,   // + 8.3 KB static
+                                                static_cast<int>(kMaxDynSmem - 12288)));
         for (const void* k : {(const void*)k_count, (const void*)k_expand<true>,
                               (const void*)k_expand<true, true>, (const void*)k_expand<false>,
                               (const void*)k_roots})
@@ -936,6 +944,7 @@ struct Engine::Impl {
         evo_frange.release(st);
         frng.release(st);
         slice_off.release(st);
+        seg_off.release(st);
         evo_new.release(st);
         ev_anc.release(st);
         ev_bmask.release(st);
@@ -962,8 +971,6 @@ struct Engine::Impl {
         rules.release(st);
         evos.release(st);
         cudaStreamSynchronize(st);
-        cudaEventDestroy(ev_a);
-        cudaEventDestroy(ev_b);
         for (auto e : ev_pool) cudaEventDestroy(e);
         cudaStreamDestroy(st);
     }
@@ -983,6 +990,7 @@ struct Engine::Impl {
         frontier_size = 0;
         ne_bound = nocc_bound = 1;
         run_ne = run_no = 1;
+        uniform = true;
         hist = LevelHist{};
         fresh_run = true;   // the next admission clears the arena top, the error flags and the counters
         times = StageTimes{};
@@ -1232,6 +1240,15 @@ struct Engine::Impl {
             }
             rm.stride = std::max<uint32_t>(rm.stride, d.rule_count);
             rm.arity = std::max<uint32_t>(rm.arity, q.arity);
+            {
+                const size_t a = spec.roots[0][0].size();
+                bool one = a == 2 || a == 3;
+                for (const auto& root : spec.roots)
+                    for (const auto& e : root) one = one && e.size() == a;
+                for (const DevRule& pr : q.rules)
+                    for (uint32_t k = 0; k < pr.n_rhs; ++k) one = one && pr.rhs_ar[k] == a;
+                uniform = uniform && one;
+            }
             max_label = std::max(max_label, q.max_label);
             const uint32_t nr = static_cast<uint32_t>(q.nes.size());
             for (uint32_t k = 0; k < nr; ++k) {
@@ -2261,7 +2278,6 @@ struct Engine::Impl {
         const uint32_t tot[6] = {uint32_t(hs[0]), uint32_t(hs[0] >> 32), uint32_t(hs[1]),
                                  uint32_t(hs[1] >> 32), uint32_t(hs[2]), uint32_t(hs[2] >> 32)};
         const uint32_t fmax_cnt = uint32_t(hs[3]);
-        const uint32_t n_warp_states = uint32_t(hs[3] >> 32);   // 0: no warp-path launches
         const uint32_t fmax_nv = uint32_t(hs[4]);                // largest frontier vertex count
         std::vector<uint32_t> h_first(nevo), h_last(nevo);
         std::vector<unsigned long long> h_classes(hs + 5, hs + 5 + nevo),
@@ -2277,6 +2293,15 @@ struct Engine::Impl {
             uint64_t(next_vertex) + n_fresh >= 0xFFFFFFF0ull || uint64_t(n_cons) + n_cons_lv >= 0xFFFFFFF0ull)
             throw std::runtime_error("hgx: 32-bit id space exhausted (events, edges or vertices)");
         A.n_events = n_ev;
+        // single-rule evolutions of one edge arity (2 or 3) each: children by the segment kernel
+        // rather than one per lane, but for the largest levels of small binary states, which fill
+        // the lanes and keep them on like work (C2's last levels, lane against segment: 7.2 against
+        // 8.6 ms; C3 2.3 against 1.4 ms, the 1,024 random evolutions 65 against 25 ms, C2's level 7
+        // -- 989,694 children -- the same)
+        const bool seg = R == 1 && uniform && !fwd &&
+                         !(rm.arity == 2 && fmax_nv + rm.fresh <= 16 && n_ev >= kLaneLevel);
+        A.path = seg ? 4u : 1u;
+        const uint32_t n_warp_states = seg ? uint32_t(hs[4] >> 32) : uint32_t(hs[3] >> 32);   // 0: no warp-path launches
 
         // capacity
         grow_events(n_events + n_ev);
@@ -2329,27 +2354,15 @@ struct Engine::Impl {
         // frontier order are cut from the level; those of the others are voided (in-range ids,
         // never kept).
         uint32_t F_eff = F;
-        bool tune = false, walk = false;   // join autotuner: measure this level / variant used
-        uint32_t bucket = 0;
         if (n_ev) {
             const uint32_t mne = std::max<uint32_t>(fmax_ne, 1), mno = std::max<uint32_t>(fmax_nocc, 1);
             const Layout Ll = make_layout(std::min<uint32_t>(mne, kLaneEMax), mno, rm, LayoutKind::Lane, fwd,
                                           fmax_cnt);
             const Layout Lw = make_layout(mne, mno, rm, LayoutKind::Warp, fwd, kLaneJoinCap,
                                           opt.join_index != 0, fmax_nv);
-            // lane kernel join: autotuned per bucket of children per frontier state (the walk
-            // amortises its count-and-emit passes over many children per state)
-            const uint64_t per_state = n_ev / std::max<uint32_t>(F, 1);
-            while (bucket < 7 && (2ull << bucket) <= per_state) ++bucket;
-            walk = per_state >= 32;
-            if (opt.lane_join == 1) walk = false;
-            else if (opt.lane_join == 2) walk = true;
-            else {
-                const uint32_t* tn = tuner.n[bucket];
-                if (tn[0] >= 1 && tn[1] >= 1) walk = tuner.ns[bucket][1] < tuner.ns[bucket][0];
-                else if (n_ev >= kTuneMinChildren) walk = tn[1] < tn[0];   // the less-sampled one
-                tune = n_ev >= kTuneMinChildren;
-            }
+            // matches by lane walks; the warp join where it is asked for (rules of more than four
+            // left-hand edges take it by themselves)
+            const bool walk = opt.lane_join != 1;
             // single-rule evolutions: batches of children cross parents (two parent regions per warp)
             Layout Ll2 = Ll;
             Ll2.bytes = Ll.bytes + (kLaneRegions - 1) * Ll.region_bytes;   // one batch per warp
@@ -2361,21 +2374,54 @@ struct Engine::Impl {
                                    : (walk ? warp_shape(k_expand<true, true>, Ll, F)
                                            : warp_shape(k_expand<true>, Ll, F));
             LaunchShape sw = warp_shape(k_expand<false>, Lw, n_ev);   // work units: slices
-            auto expand = [&](uint32_t n_work) {
+            // segment kernel: 16 lanes a child when every child of the level has at most 16 vertices;
+            // at most 64 children a work unit, fewer (down to one) where that would leave warps of
+            // the launch without work: a unit's children are hashed one after another, 10-25 us each
+            const uint32_t S = fmax_nv + rm.fresh <= 16 ? 16 : 32;
+            auto slice_for = [&](uint64_t events) {
+                uint32_t s = 64;
+                while (s > 1 && events / s < kNumSMs * 24) s >>= 1;
+                return s;
+            };
+            A.slice = slice_for(n_ev);
+            Layout Ls;
+            if (seg) {
+                const uint32_t ne = std::min<uint32_t>(mne, kLaneEMax);
+                Ls = make_layout(ne, std::min<uint32_t>(mno, ne * rm.arity), rm, LayoutKind::Seg, false, 64,
+                                 false, std::min<uint32_t>(fmax_nv, kLaneVMax), S);
+                const uint64_t units = uint64_t(F) + n_ev / A.slice;
+                sl = S == 16 ? (walk ? warp_shape(k_expand_seg<16, true>, Ls, units) : warp_shape(k_expand_seg<16, false>, Ls, units))
+                             : (walk ? warp_shape(k_expand_seg<32, true>, Ls, units) : warp_shape(k_expand_seg<32, false>, Ls, units));
+            }
+            auto expand = [&](uint32_t n_work, uint64_t n_children) {
                 A.f_begin = 0;
                 A.f_end = n_work;
                 HGX_CUDA_CHECK(cudaMemsetAsync(work.p + 1, 0, 2 * sizeof(uint32_t), st));
                 tic(true);
-                if (tune) HGX_CUDA_CHECK(cudaEventRecord(ev_a, st));
+                if (seg) {
+                    A.slice = slice_for(n_children);
+                    if (fmax_cnt > A.slice) {
+                        seg_off.ensure(uint64_t(n_work) + 1, 0, st);
+                        k_seg_slices<<<grid_for(n_work, 256), 256, 0, st>>>(A, n_work, seg_off.p);
+                        check_launch();
+                        scan(seg_off.p, seg_off.p, n_work);
+                        A.soff = seg_off.p;
+                        A.n_sw = n_work;
+                    }
+                    if (S == 16 && walk) k_expand_seg<16, true><<<sl.grid, sl.block, sl.smem, st>>>(ptrs(), A, Ls);
+                    else if (S == 16) k_expand_seg<16, false><<<sl.grid, sl.block, sl.smem, st>>>(ptrs(), A, Ls);
+                    else if (walk) k_expand_seg<32, true><<<sl.grid, sl.block, sl.smem, st>>>(ptrs(), A, Ls);
+                    else k_expand_seg<32, false><<<sl.grid, sl.block, sl.smem, st>>>(ptrs(), A, Ls);
+                    A.soff = nullptr;
+                }
                 // levels without forwarding run the lane kernel compiled without its paths
-                if (cross && walk && fwd) k_expand_lanes2<true, kLaneRegions><<<sl.grid, sl.block, sl.smem, st>>>(ptrs(), A, Ll);
+                else if (cross && walk && fwd) k_expand_lanes2<true, kLaneRegions><<<sl.grid, sl.block, sl.smem, st>>>(ptrs(), A, Ll);
                 else if (cross && walk) k_expand_lanes2<true, kLaneRegions, false><<<sl.grid, sl.block, sl.smem, st>>>(ptrs(), A, Ll);
                 else if (cross && fwd) k_expand_lanes2<false, kLaneRegions><<<sl.grid, sl.block, sl.smem, st>>>(ptrs(), A, Ll);
                 else if (cross) k_expand_lanes2<false, kLaneRegions, false><<<sl.grid, sl.block, sl.smem, st>>>(ptrs(), A, Ll);
                 else if (walk) k_expand<true, true><<<sl.grid, sl.block, sl.smem, st>>>(ptrs(), A, Ll);
                 else k_expand<true><<<sl.grid, sl.block, sl.smem, st>>>(ptrs(), A, Ll);
                 check_launch();
-                if (tune) HGX_CUDA_CHECK(cudaEventRecord(ev_b, st));
                 toc(times.expand, true);
                 ++times.expand_launches;
                 if (walk) ++times.walk_launches;
@@ -2410,13 +2456,12 @@ struct Engine::Impl {
             }
             if (capped.empty() || avoidable < opt.chunk_min) {
                 A.frng = nullptr;
-                expand(F);
+                expand(F, n_ev);
                 tic();
                 k_select<<<grid_for(n_ev, 256), 256, 0, st>>>(ptrs(), A, 0, n_ev);
                 check_launch();
                 toc(times.select);
             } else {
-                tune = false;   // rounds: several launches, no single measurement window
                 std::vector<uint32_t> h_item(NI + 1), h_fr(2 * nevo);
                 readback(h_item.data(), item_ev.p, (NI + 1) * 4);
                 readback(h_fr.data(), evo_frange.p, 2 * nevo * 4);
@@ -2431,6 +2476,9 @@ struct Engine::Impl {
                 // the frontier ranges of a round, merged where adjacent, uploaded as A.frng
                 std::vector<std::pair<uint32_t, uint32_t>> rng;
                 auto run_ranges = [&](bool select) -> uint32_t {
+                    uint64_t n_round = 0;   // children of the round
+                    for (const auto& r : rng)
+                        if (r.first < r.second) n_round += fev(r.second) - fev(r.first);
                     std::sort(rng.begin(), rng.end());
                     std::vector<uint32_t> lo, off(1, 0);
                     for (const auto& r : rng) {
@@ -2452,7 +2500,7 @@ struct Engine::Impl {
                     A.frng = frng.p;
                     A.n_frng = n;
                     if (select) {
-                        expand(total);
+                        expand(total, n_round);
                         tic();
                         k_select_list<<<grid_for(uint64_t(total) * 32, 256), 256, 0, st>>>(ptrs(), A, total, evo_new.p);
                         check_launch();
@@ -2598,15 +2646,6 @@ struct Engine::Impl {
         }
         const std::vector<uint32_t> h_rng(hs2, hs2 + 7 * nevo);
         const uint32_t* s2 = hs2 + 7 * nevo;
-        if (tune) {
-            float ms = 0;
-            HGX_CUDA_CHECK(cudaEventElapsedTime(&ms, ev_a, ev_b));
-            const double x = double(ms) * 1e6 / double(n_ev);
-            double& avg = tuner.ns[bucket][walk ? 1 : 0];
-            uint32_t& cnt = tuner.n[bucket][walk ? 1 : 0];
-            avg = cnt ? 0.75 * avg + 0.25 * x : x;
-            ++cnt;
-        }
         if (s2[3] & kErrTrDepth)
             throw std::invalid_argument("transitive reduction supports evolutions of at most 64 levels");
         if (s2[3]) throw std::runtime_error("hgx: device error flags 0x" + std::to_string(s2[3]));
@@ -2889,31 +2928,115 @@ __global__ void k_noalloc_classes(DevPtrs P, DevEvo ev, const uint64_t* hash, ui
         cls[i] = table_lookup(P, ev, hash[i]);
 }
 
-// Warp per state: WL hash into hash[i], then insert (hash, i) into the table (smallest i wins).
-__global__ void __launch_bounds__(256) k_noalloc_hash(DevPtrs P, DevEvo ev, uint32_t n,
-                                                     uint32_t* work, uint64_t* hash, Layout L) {
+// States of at most 32 vertices and 64 edges of one arity (2 or 3), a warp each: the record's arities
+// are checked and its vertices numbered through a 128-slot table, then the segment hash (seg_wl.cuh).
+// Every other state is marked in cls[i] and counted, for k_noalloc_hash. 3 KB of shared memory a warp
+// in place of 13 (whose neighbour buffer has to allow arity 16), and a quarter of the instructions:
+// 200,003 states of 4-40 edges 3.46 -> 0.83 ms.
+__global__ void __launch_bounds__(256, 4) k_noalloc_seg(DevPtrs P, DevEvo ev, uint32_t n, uint32_t max_edges,
+                                                       uint32_t max_occ, uint32_t* counters, uint64_t* hash,
+                                                       uint32_t* cls, uint32_t ne_cap, uint32_t listn,
+                                                       uint32_t bytes) {
     extern __shared__ __align__(16) char smem[];
-    char* sm = smem + (threadIdx.x >> 5) * L.bytes;
+    constexpr uint32_t full = 0xFFFFFFFFu, TS = 128;
+    __shared__ SegTables tables;
+    seg_tables_fill(tables);
+    char* scr = smem + (threadIdx.x >> 5) * bytes;
+    uint32_t* tab = reinterpret_cast<uint32_t*>(scr + align_up(seg_scratch_bytes(32, ne_cap, listn), 16));
+    uint8_t* tid = reinterpret_cast<uint8_t*>(tab + TS);
+    uint8_t* slot = tid + TS;                         // table slot, then local id, of each occurrence
     const uint32_t lane = lane_id();
-    while (true) {
-        uint32_t i = 0;
-        if (lane == 0) i = atomicAdd(work, 1u);
-        i = __shfl_sync(0xFFFFFFFFu, i, 0);
-        if (i >= n) break;
-        const Parent pa = load_parent(P, L, sm, i);
-        uint8_t* car = smp<uint8_t>(sm, L.o_car);
-        uint16_t* cvo = smp<uint16_t>(sm, L.o_cvo);
-        const uint8_t* pear = smp<uint8_t>(sm, L.o_pear);
-        const uint16_t* pevo = smp<uint16_t>(sm, L.o_pevo);
-        for (uint32_t e = lane; e < pa.ne; e += 32) { car[e] = pear[e]; cvo[e] = pevo[e]; }
-        __syncwarp();
+    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+    for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += warps) {
+        const uint32_t ne = P.st_ne[i], nocc = P.st_nocc[i];
+        const uint32_t* rec = P.arena + P.st_off[i];
+        bool ok = ne >= 1 && ne <= ne_cap && nocc <= max_occ && (nocc == 2 * ne || nocc == 3 * ne);
+        const uint32_t A = ok ? nocc / ne : 0u;
+        if (ok) {
+            const uint32_t aw = (ne + 3) >> 2;
+            for (uint32_t k = lane; k < ne; k += 32) ok = ok && ((rec[ne + (k >> 2)] >> ((k & 3u) * 8u)) & 0xFFu) == A;
+            for (uint32_t t = lane; t < TS; t += 32) tab[t] = kNone;
+            __syncwarp();
+            for (uint32_t j = lane; j < nocc; j += 32) {
+                const uint32_t v = rec[ne + aw + j];
+                uint32_t h = (v * 2654435761u) >> 25;
+                bool placed = false;
+                for (uint32_t probe = 0; probe < TS && v != kNone; ++probe) {
+                    const uint32_t prev = atomicCAS(&tab[h], kNone, v);
+                    if (prev == kNone || prev == v) { placed = true; break; }
+                    h = (h + 1) & (TS - 1);
+                }
+                ok = ok && placed;
+                slot[j] = static_cast<uint8_t>(h);
+            }
+            __syncwarp();
+            uint32_t ids = 0;
+            for (uint32_t b = 0; b < TS; b += 32) {
+                const bool used = tab[b + lane] != kNone;
+                const uint32_t bal = __ballot_sync(full, used);
+                if (used) tid[b + lane] = static_cast<uint8_t>(ids + __popc(bal & ((1u << lane) - 1u)));
+                ids += __popc(bal);
+            }
+            __syncwarp();
+            for (uint32_t j = lane; j < nocc; j += 32) slot[j] = tid[slot[j]];
+            __syncwarp();
+            ok = ok && ids <= 32;
+        }
+        if (!__all_sync(full, ok)) {   // warp-uniform
+            if (lane == 0) {
+                cls[i] = kNone;
+                atomicAdd(&counters[2], 1u);
+            }
+            __syncwarp();
+            continue;
+        }
         WlInfo info;
-        const uint64_t h = warp_wl(L, sm, pa.ne, pa.nvp, info);
+        const uint64_t h = seg_wl<32>(ne, 32, A, false, scr, ne_cap, listn, tables, [&](uint32_t k) -> uint32_t {
+            const uint8_t* s = slot + k * A;
+            return s[0] | (uint32_t(s[1]) << 8) | (A == 3 ? uint32_t(s[2]) << 16 : 0u);
+        }, info);
         if (lane == 0) {
             hash[i] = h;
+            cls[i] = 0;
             table_insert(P, ev, h, i);
         }
         __syncwarp();
+    }
+}
+
+// Warp per state that k_noalloc_seg marked: WL hash into hash[i], then insert (hash, i) into the
+// table (smallest i wins).
+__global__ void __launch_bounds__(256) k_noalloc_hash(DevPtrs P, DevEvo ev, uint32_t n,
+                                                     uint32_t* counters, uint64_t* hash,
+                                                     const uint32_t* cls, Layout L) {
+    extern __shared__ __align__(16) char smem[];
+    char* sm = smem + (threadIdx.x >> 5) * L.bytes;
+    const uint32_t lane = lane_id();
+    if (counters[2] == 0) return;
+    // 32 states a grab: their marks in one load, the marked ones one after another
+    while (true) {
+        uint32_t i0 = 0;
+        if (lane == 0) i0 = atomicAdd(&counters[0], 32u);
+        i0 = __shfl_sync(0xFFFFFFFFu, i0, 0);
+        if (i0 >= n) break;
+        uint32_t todo = __ballot_sync(0xFFFFFFFFu, i0 + lane < n && cls[i0 + lane] == kNone);
+        for (; todo; todo &= todo - 1) {
+            const uint32_t i = i0 + __ffs(todo) - 1;
+            const Parent pa = load_parent(P, L, sm, i);
+            uint8_t* car = smp<uint8_t>(sm, L.o_car);
+            uint16_t* cvo = smp<uint16_t>(sm, L.o_cvo);
+            const uint8_t* pear = smp<uint8_t>(sm, L.o_pear);
+            const uint16_t* pevo = smp<uint16_t>(sm, L.o_pevo);
+            for (uint32_t e = lane; e < pa.ne; e += 32) { car[e] = pear[e]; cvo[e] = pevo[e]; }
+            __syncwarp();
+            WlInfo info;
+            const uint64_t h = warp_wl(L, sm, pa.ne, pa.nvp, info);
+            if (lane == 0) {
+                hash[i] = h;
+                table_insert(P, ev, h, i);
+            }
+            __syncwarp();
+        }
     }
 }
 
@@ -2957,6 +3080,9 @@ extern "C" HGX_API hgx_status hgx_hash_states_noalloc(
                 HGX_CUDA_CHECK(cudaFuncSetAttribute(k_noalloc_hash,
                                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                     static_cast<int>(kMaxDynSmem)));
+                HGX_CUDA_CHECK(cudaFuncSetAttribute(k_noalloc_seg,   // + 6 KB static
+                                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                    static_cast<int>(kMaxDynSmem - 8192)));
                 g_noalloc_ptr[dev] = p;
             }
             base = static_cast<unsigned char*>(g_noalloc_ptr[dev]);
@@ -2976,7 +3102,7 @@ extern "C" HGX_API hgx_status hgx_hash_states_noalloc(
         // slots [0, cap) plus the key-0 slot at index cap
         HGX_CUDA_CHECK(cudaMemsetAsync(keys, 0, (cap + 1) * 8, st));
         HGX_CUDA_CHECK(cudaMemsetAsync(vals, 0xFF, (cap + 1) * 4, st));
-        HGX_CUDA_CHECK(cudaMemsetAsync(counters, 0, 8, st));
+        HGX_CUDA_CHECK(cudaMemsetAsync(counters, 0, 16, st));
         DevPtrs P;
         std::memset(&P, 0, sizeof(P));
         P.arena = const_cast<uint32_t*>(d_records);
@@ -2988,7 +3114,14 @@ extern "C" HGX_API hgx_status hgx_hash_states_noalloc(
         P.err = counters + 1;
         const uint32_t wpb = static_cast<uint32_t>(std::min<size_t>(8, std::max<size_t>(1, (96 * 1024) / L.bytes)));
         const uint32_t grid = static_cast<uint32_t>(std::min<uint64_t>((n_states + wpb - 1) / wpb, kNumSMs * 4));
-        k_noalloc_hash<<<grid, 32 * wpb, L.bytes * wpb, st>>>(P, ev, n_states, counters, d_hash, L);
+        const uint32_t ne_cap = std::min<uint32_t>(max_edges, kSegEMax);
+        const uint32_t listn = std::max<uint32_t>(2 * ne_cap, std::min<uint32_t>(6 * ne_cap, 2 * std::min<uint32_t>(max_occ, 3 * kSegEMax)));
+        const uint32_t sb = align_up(align_up(seg_scratch_bytes(32, ne_cap, listn), 16) + 128 * 5 + 3 * kSegEMax, 16);
+        const uint32_t sgrid = static_cast<uint32_t>(std::min<uint64_t>((n_states + 7) / 8, kNumSMs * 4));
+        k_noalloc_seg<<<sgrid, 256, sb * 8, st>>>(P, ev, n_states, max_edges, max_occ, counters, d_hash, d_class,
+                                                  ne_cap, listn, sb);
+        HGX_CUDA_CHECK(cudaGetLastError());
+        k_noalloc_hash<<<grid, 32 * wpb, L.bytes * wpb, st>>>(P, ev, n_states, counters, d_hash, d_class, L);
         HGX_CUDA_CHECK(cudaGetLastError());
         k_noalloc_classes<<<(n_states + 255) / 256, 256, 0, st>>>(P, ev, d_hash, n_states, d_class);
         HGX_CUDA_CHECK(cudaGetLastError());

@@ -99,8 +99,8 @@ struct RunOptions {
     // Event canonicalisation: hgcommon EventSignatureKeys bits 0-3 (input state, output state,
     // step, rule); 0 = every application is its own event.
     uint32_t event_keys = 0;
-    // Join of the lane (small-state) expand kernel: 0 = autotuned per bucket of children per
-    // frontier state, 1 = warp join, 2 = lane-parallel walk. Results are identical.
+    // Join of the small-state expand kernels: 0 or 2 = lane-parallel walk, 1 = warp join. Results
+    // are identical.
     uint32_t lane_join = 0;
     // Capped single evolution: 0 = split a level at the estimated cut, 1 = never, N >= 2 = at N.
     uint64_t level_split = 0;

@@ -205,13 +205,14 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_levels(DevPtrs P, FusedArg
                 const uint32_t sid = frontier[f];
                 const Parent pa = load_parent(P, L, sm, sid);
                 build_join_index(L, sm, pa);
+                const unsigned long long* vm = build_vmask(L, sm, pa);
                 const DevEvo ev = P.evos[P.st_evo[sid]];
                 unsigned long long c_all = 0;
                 for (uint32_t r = 0; r < R; ++r) {
                     uint32_t cnt = 0;
                     if (r < ev.rule_count) {
                         load_rule(sm, L, &P.rules[ev.rule_begin + r]);
-                        if (pa.ne <= kLaneEMax && Rr.n_lhs <= kLaneJoinLhs) cnt = lane_join_count(L, sm, Rr, pa);
+                        if (pa.ne <= kLaneEMax && Rr.n_lhs <= kLaneJoinLhs) cnt = lane_join_count(L, sm, Rr, pa, vm);
                         else warp_join(L, sm, Rr, pa, Rr.sched, -1, [&](uint32_t) { ++cnt; }, 0xFFFFFFFFu,
                                        SkipCounter{&cnt, 0xFFFFFFFFu});
                     }
@@ -335,6 +336,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_levels(DevPtrs P, FusedArg
             uint32_t staged = kNone;
             Parent pa{0, 0, 0};
             bool pconn = false;
+            const unsigned long long* vm = nullptr;
             for (uint32_t t = lo_t, x = x0; x < x1; ++t) {
                 const uint32_t t0 = G.item_ev[t], rn = G.cnt[t];
                 if (x >= t0 + rn) continue;   // an item without events
@@ -346,6 +348,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_levels(DevPtrs P, FusedArg
                     pa = load_parent(P, L, sm, sid);
                     build_join_index(L, sm, pa);
                     pconn = parent_connected(L, sm, pa);
+                    vm = build_vmask(L, sm, pa);
                     if (lane == 0 && t0 == x) b_hbm += 4ull * (pa.ne + (pa.ne + 3) / 4 + pa.nocc) + 20;
                 }
                 load_rule(sm, L, &P.rules[ev.rule_begin + r]);
@@ -396,11 +399,11 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_levels(DevPtrs P, FusedArg
                         uint32_t done = 0;
                         for (uint32_t e0b = 0; e0b < pa.ne; e0b += 32) {
                             const uint32_t e0 = e0b + lane;
-                            const uint32_t c = e0 < pa.ne ? lane_walk(L, sm, Rr, pa, e0, [](uint32_t) {}) : 0u;
+                            const uint32_t c = e0 < pa.ne ? lane_walk(L, sm, Rr, pa, e0, vm, [](uint32_t) {}) : 0u;
                             const uint32_t inc = warp_incl_scan(c);
                             uint32_t at = done + inc - c;
                             if (c && at < s1 && at + c > s0)
-                                lane_walk(L, sm, Rr, pa, e0, [&](uint32_t pk) {
+                                lane_walk(L, sm, Rr, pa, e0, vm, [&](uint32_t pk) {
                                     if (at >= s0 && at < s1) list[at - s0] = pk;
                                     ++at;
                                 });

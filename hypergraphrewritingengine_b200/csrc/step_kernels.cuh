@@ -101,10 +101,13 @@ struct LevelArgs {
     // counts (soff[n_sw] = total); a slice is a run of slice_size(children) consecutive children
     const uint32_t* soff;
     uint32_t n_sw;
-    uint8_t* fmode;             // [F] bit 0: children hashed lane-per-child; bit 1: forwarding
+    uint8_t* fmode;             // [F] bit 0: within the lane path's limits; bit 1: forwarding;
+                                // bit 2: within the segment path's
     uint32_t fwd_mode;          // 0 off, 1 every eligible state, 2 states with >= 48 edges
     uint32_t ev_keys;           // event signature keys (0 = no event canonicalisation)
     uint32_t lane_vmax;         // largest child (vertices) of this level the lane path takes
+    uint32_t path;              // the level's small-state kernel as its fmode bit: 1 lane, 4 segment
+    uint32_t slice;             // segment kernel: most children of a work unit
     uint32_t* work;             // work-queue counters
     // select / assign
     uint32_t* flag_new;         // [n_events]
@@ -149,11 +152,15 @@ struct Layout {
     // sorted copy), a 32-match chunk of forwarded matches
     uint32_t o_sched2, o_fkc, o_dkey, o_dpos, o_dkey2, o_dpos2, o_fkey, o_fpos;
     uint32_t SB;                                                    // bytes per batch slot
+    // segment path: packed parent edges, per-segment scratch for states of at most SEGE edges and
+    // SEGN neighbour entries, produced edges per batch slot
+    uint32_t o_ppk, o_seg, SEGB, SEGE, SEGN, RHS;
     uint32_t VT, o_vtab, o_vtid;   // vertex hash table for large states (VT slots, 0 = unused)
     uint32_t o_srt;                // warp WL: sort buffer of the distinct-colour count
     // join indices of a staged state past kJoinIndexMin edges (XI = 1; count and warp layouts):
     // vertex -> state positions of the edges holding it (CSR), and the edges bucketed by
     // signature (at most kSigBuckets buckets); o_xready: bit 0 vertex index, bit 1 signature index
+    uint32_t VM, o_vm;             // edge masks by vertex (lane walks): room for VM vertices
     uint32_t XI, o_xready, o_xoff, o_xinc, o_bkey, o_boff, o_blist;
     uint32_t bytes;
 };

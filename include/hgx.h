@@ -92,9 +92,8 @@ typedef enum hgx_option {
        reference. The edge-rank keys (16, 32; the Automatic preset) need an exact canonical
        labelling of every state and are rejected. Default 0. */
     HGX_OPT_EVENT_SIGNATURE_KEYS = 10,
-    /* Join of the small-state expand kernel: 0 (default) = chosen per level by the engine's
-       autotuner (device time per child, per bucket of children per frontier state), 1 = warp join,
-       2 = lane-parallel walk. No reference counterpart; results are identical. */
+    /* Join of the small-state expand kernels: 0 (default) and 2 = lane-parallel walk, 1 = warp
+       join. No reference counterpart; results are identical. */
     HGX_OPT_LANE_JOIN = 11,
     /* A single evolution under a state cap: a level whose cut the previous level's ratios place
        early in its frontier is counted and expanded as a frontier prefix first, the rest only if
@@ -264,7 +263,7 @@ HGX_API hgx_status hgx_engine_stage_times(hgx_engine* engine, double* out_ms, ui
    WL + dedup counted as separate HBM streams), bytes the fused kernel itself must move to or
    from HBM, children hashed, WL refinement rounds, launches. out[5..8], warp-per-child kernel:
    the same first four figures; out[9] its total device time in nanoseconds; out[10] lane-kernel
-   launches that ran the lane-parallel walk (the join autotuner's choice; out has 11 entries). */
+   launches that ran the lane-parallel walk (out has 11 entries). */
 HGX_API hgx_status hgx_engine_expand_stats(hgx_engine* engine, uint64_t* out);
 
 /* The last evolve call's result: out[0] = 1 if it was streamed (copied to the host range by
