@@ -61,8 +61,10 @@ constexpr uint32_t kHashOccMin = 96;
 
 // Join indices: states of more than kJoinIndexMin edges staged for the warp join carry a vertex
 // index and, when their edges fall in at most kSigBuckets signatures, a signature index.
-constexpr uint32_t kJoinIndexMin = 96;
+constexpr uint32_t kJoinIndexMin = 64;
 constexpr uint32_t kSigBuckets = 16;
+// Large states (up to 32 kChunks edges): matches counted per 32 first edges.
+constexpr uint32_t kChunks = 16;
 
 // (Writing the multiply by the prime 2^40 + 0x1b3 as a shift and a 32-bit multiply measured
 // slower on the lane expand kernel: 6.72 -> 6.79 ms per C2 evolution.)

@@ -180,6 +180,9 @@ constexpr uint32_t kLaneLevel = 1u << 20;
 // shorter than the per-range work streaming adds).
 constexpr uint64_t kStreamMinBytes = 64ull << 20;
 
+// Matches listed at a time by the warp path, and neighbour words of its WL rounds in shared memory.
+constexpr uint32_t kListMax = 32, kWlBuf = 640;
+
 enum class LayoutKind { Count, Lane, Warp, Seg };
 
 // Shared-memory carve-up per warp. Count: the parent and the join. Lane: plus the parent's
@@ -196,13 +199,11 @@ __host__ __device__ Layout make_layout(uint32_t NE, uint32_t NOCC, const RuleMax
     NOCC = std::max<uint32_t>(NOCC, 1);
     L.NE = NE;
     L.NOCC = NOCC;
-    L.CNE = NE + rm.rhs;
+    L.CNE = NE + rm.rhs;   // (at most 4,095 edges: see warp_shape)
     L.CNOCC = NOCC + rm.rhs_total;
     L.NV = NV ? std::min(std::max<uint32_t>(NV, 1), NOCC) : NOCC;
     L.V = L.NV + rm.fresh;
     L.W = (NE + 31) / 32;
-    // neighbour-sort entries of one WL round: sum over occurrences of max(a - 1, 1)
-    L.NBR = wl ? L.CNOCC * std::max<uint32_t>(rm.arity - 1, 1) : 0;
     uint32_t off = 0;
     auto take = [&](uint32_t bytes, uint32_t align) {
         off = align_up(off, align);
@@ -210,31 +211,19 @@ __host__ __device__ Layout make_layout(uint32_t NE, uint32_t NOCC, const RuleMax
         off += bytes;
         return o;
     };
-    if (wl) {
-        L.o_cur = take(8 * L.V, 8);
-        L.o_nxt = take(8 * L.V, 8);
-        L.o_csum = take(8 * L.V, 8);
-        L.o_ccnt = take(8 * L.V, 8);
-        L.o_nbr = take(8 * L.NBR, 8);
-    }
+    // what a staged state keeps for all of its work
     L.o_peid = take(4 * NE, 4);
-    L.o_occ = take(4 * (wl ? L.CNOCC : NOCC), 4);
-    L.o_deg = take(4 * (wl ? std::max(L.V, NOCC) : NOCC), 4);   // also load_parent's first-occurrence scratch
-    if (wl) {
-        L.o_ooff = take(4 * (L.V + 1), 4);
-        L.o_nbo = take(4 * (L.V + 1), 4);
-        L.o_nn = take(4 * L.V, 4);
-        L.o_comp = take(4 * L.V, 4);
-    }
-    L.o_cand = take(4 * kMaxPatternEdges * L.W, 4);
     L.o_taken = take(4 * L.W, 4);
     L.o_misc = take(4 * kMaxPatternEdges, 4);
+    L.o_xready = take(4, 4);
     L.o_pevo = take(2 * NE, 2);
     L.o_vloc = take(2 * (NOCC + rm.rhs_total), 2);
     if (wl) L.o_cvo = take(2 * L.CNE, 2);
     L.o_bind = take(2 * kMaxVars, 2);
     L.o_match = take(2 * kMaxPatternEdges, 2);
     L.o_mdepth = take(2 * kMaxPatternEdges, 2);
+    L.LH = rm.lhs;
+    if (wl) L.o_mpos = take(2 * rm.lhs * kListMax, 2);
     L.o_pear = take(NE, 1);
     if (wl) L.o_car = take(L.CNE, 1);
     L.o_rule = take(sizeof(DevRule), 4);
@@ -248,17 +237,29 @@ __host__ __device__ Layout make_layout(uint32_t NE, uint32_t NOCC, const RuleMax
         L.o_fpos = take(2 * kFwdMaxLhs * 32, 2);
         L.o_sched2 = take(kMaxPatternEdges, 1);
     }
+    // one after another in the same bytes: load_parent's scratch; the join (candidates, indices);
+    // the WL arrays of one child
+    const uint32_t u0 = align_up(off, 8);
+    uint32_t u1 = u0;
+    auto next_use = [&] {
+        u1 = std::max(u1, off);
+        off = u0;
+    };
+    off = u0;
+    L.o_glob = take(4 * NOCC, 4);
+    L.o_first = take(4 * NOCC, 4);
     if (NOCC > kHashOccMin) {
         L.VT = 64;   // load <= 1/2 over the state's distinct vertices
         while (L.VT < 2 * L.NV) L.VT <<= 1;
         L.o_vtab = take(4 * L.VT, 4);
         L.o_vtid = take(2 * L.VT, 2);
     }
-    L.VM = std::min<uint32_t>(L.NV, kind == LayoutKind::Lane || kind == LayoutKind::Seg ? kLaneVMax : 64);
+    if (!lane) next_use();   // (the lane layouts go on using the scratch)
+    L.o_cand = take(4 * kMaxPatternEdges * L.W, 4);
+    L.VM = std::min<uint32_t>(L.NV, lane ? kLaneVMax : 64);
     L.o_vm = take(8 * L.VM, 8);
     if (index && !lane && NE > kJoinIndexMin) {
         L.XI = 1;
-        L.o_xready = take(4, 4);
         L.o_xoff = take(4 * (NOCC + 1), 4);
         L.o_xinc = take(2 * NOCC, 2);
         L.o_bkey = take(8 * (kSigBuckets + 1), 8);
@@ -266,9 +267,25 @@ __host__ __device__ Layout make_layout(uint32_t NE, uint32_t NOCC, const RuleMax
         L.o_blist = take(2 * NE, 2);
     }
     if (wl) {
-        uint32_t n2 = 64;   // distinct-colour hash set: >= 2 slots per vertex, + a zero flag
+        next_use();
+        L.o_cur = take(8 * L.V, 8);
+        L.o_nxt = take(8 * L.V, 8);
+        L.o_occ = take(2 * L.CNOCC, 4);
+        L.o_deg = take(4 * L.V, 4);
+        L.o_nn = take(4 * L.V, 4);
+        L.o_ooff = take(4 * L.V, 4);
+        L.o_comp = take(4 * L.V, 4);
+        // neighbour words: every vertex's at once if they are few, else as many vertices at a time as
+        // fit kWlBuf words; between the rounds the distinct-colour hash set (two slots per vertex and
+        // a zero flag), after them the per-component sums
+        uint32_t n2 = 64;
         while (n2 < 2 * L.V) n2 <<= 1;
-        L.o_srt = take(8 * (n2 + 1), 8);
+        L.BUF = std::max<uint32_t>(std::min<uint32_t>(L.CNOCC * std::max<uint32_t>(rm.arity - 1, 1), +kWlBuf), n2 + 1);
+        L.o_buf = take(8 * L.BUF, 8);
+    }
+    if (!lane) {
+        next_use();
+        off = u1;
     }
     if (kind == LayoutKind::Seg) {
         L.o_ppk = take(4 * NE, 4);
@@ -450,7 +467,7 @@ struct Engine::Impl {
     DVec<uint32_t> bcount, boff, bpairs, scan_sums, sync_buf, root_ids;
     DVec<unsigned long long> stats, totals;
     DVec<uint8_t> fmode, fin;
-    DVec<uint32_t> fin_cnt, evo_frange, fin_ids, map_s, map_e, frng, slice_off, seg_off;
+    DVec<uint32_t> fin_cnt, evo_frange, fin_ids, map_s, map_e, frng, slice_off, seg_off, chunks;
     DVec<unsigned long long> evo_new, ev_anc, ev_sig, evo_sigs;
     DVec<unsigned long long> ev_bmask;
     DVec<uint64_t> fin_rng;
@@ -945,6 +962,7 @@ struct Engine::Impl {
         frng.release(st);
         slice_off.release(st);
         seg_off.release(st);
+        chunks.release(st);
         evo_new.release(st);
         ev_anc.release(st);
         ev_bmask.release(st);
@@ -1111,7 +1129,7 @@ struct Engine::Impl {
 
     template <class K>
     LaunchShape warp_shape(K kernel, const Layout& L, uint64_t items) {
-        if (L.bytes > kMaxDynSmem)
+        if (L.bytes > kMaxDynSmem || L.CNE > 4095)
             throw std::runtime_error("hgx: a state exceeds the per-warp shared-memory capacity (" +
                                      std::to_string(L.bytes) + " bytes needed)");
         uint32_t wpb = static_cast<uint32_t>(std::min<size_t>(8, std::max<size_t>(1, (96 * 1024) / L.bytes)));
@@ -1959,7 +1977,12 @@ struct Engine::Impl {
         uint32_t done = 0;
         bool grown = false;
         while (done < most && frontier_size) {
-            if (uint64_t(frontier_size) * rm.stride > kFusedItems) break;
+            // not worth a look: too many items, or more events than the limit to expect (each state of
+            // E edges has about E matches or more: a batch's large roots would be counted in vain), or
+            // by the last level's events per state
+            if (uint64_t(frontier_size) * rm.stride > kFusedItems || uint64_t(frontier_size) * ne_bound > 2 * kFusedEvents ||
+                (nevo == 1 && hist.valid && hist.ev_per_state * frontier_size > kFusedEvents))
+                break;
             const uint32_t levels = std::min<uint32_t>({most - done, kFusedLevels,
                                                         std::max<uint32_t>(1, static_cast<uint32_t>(4096 / nevo))});
             const size_t words = kReportWords + kFusedLevels * kLevelWords + size_t(levels) * nevo * kRangeWords;
@@ -2246,7 +2269,15 @@ struct Engine::Impl {
                                       opt.join_index != 0);
         fmode.ensure(F, 0, st);
         A.fmode = fmode.p;
-        LaunchShape sc = warp_shape(k_count, Lc, F);
+        if (ne_bound > uint32_t(kLaneEMax)) {
+            chunks.ensure(items * kChunks, 0, st);
+            A.chunks = chunks.p;
+        }
+        // large states are counted by several warps each while there are few of them: a 256-edge state
+        // with three left-hand edges is milliseconds of one warp's walks
+        A.parts = A.chunks && !fwd && F < kLaneFullStates ? std::min<uint32_t>((ne_bound + 31) / 32, 8) : 1;
+        if (A.parts > 1) HGX_CUDA_CHECK(cudaMemsetAsync(counts.p, 0, items * 4, st));
+        LaunchShape sc = warp_shape(k_count, Lc, uint64_t(F) * A.parts);
         tic();
         k_count<<<sc.grid, sc.block, sc.smem, st>>>(ptrs(), A, Lc);
         check_launch();
@@ -2373,7 +2404,7 @@ struct Engine::Impl {
                                                   : warp_shape(k_expand_lanes2<false, kLaneRegions, false>, Ll2, F)))
                                    : (walk ? warp_shape(k_expand<true, true>, Ll, F)
                                            : warp_shape(k_expand<true>, Ll, F));
-            LaunchShape sw = warp_shape(k_expand<false>, Lw, n_ev);   // work units: slices
+            LaunchShape sw = warp_shape(k_expand<false>, Lw, n_ev);   // work units: slices of children
             // segment kernel: 16 lanes a child when every child of the level has at most 16 vertices;
             // at most 64 children a work unit, fewer (down to one) where that would leave warps of
             // the launch without work: a unit's children are hashed one after another, 10-25 us each
@@ -2394,6 +2425,8 @@ struct Engine::Impl {
                              : (walk ? warp_shape(k_expand_seg<32, true>, Ls, units) : warp_shape(k_expand_seg<32, false>, Ls, units));
             }
             auto expand = [&](uint32_t n_work, uint64_t n_children) {
+                // (a share of the children takes the warp path; one child is 20-100 us of a warp)
+                A.wslice = std::min<uint32_t>(slice_for(n_children / 4), kListMax);
                 A.f_begin = 0;
                 A.f_end = n_work;
                 HGX_CUDA_CHECK(cudaMemsetAsync(work.p + 1, 0, 2 * sizeof(uint32_t), st));
@@ -2611,7 +2644,7 @@ struct Engine::Impl {
             tic();
             k_bpairs<false><<<grid_for(uint64_t(F_eff) * 32, 256), 256, 0, st>>>(ptrs(), A);
             check_launch();
-            if (fmax_ne > 63) {   // parents without position masks
+            if (fmax_ne > 63) {
                 k_bpairs_walk<false><<<grid_for(ne2, 256), 256, 0, st>>>(ptrs(), A);
                 check_launch();
             }
@@ -3062,7 +3095,7 @@ extern "C" HGX_API hgx_status hgx_hash_states_noalloc(
         RuleMax rm;
         rm.arity = kMaxArity;
         const Layout L = make_layout(max_edges, max_occ, rm, LayoutKind::Warp);
-        if (L.bytes > kMaxDynSmem)
+        if (L.bytes > kMaxDynSmem || L.CNE > 4095)
             return noalloc_fail(HGX_ERR_CAPACITY,
                                 "hgx_hash_states_noalloc: states of this size exceed shared memory");
         int dev = 0;

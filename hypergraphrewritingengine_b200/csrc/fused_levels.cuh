@@ -36,7 +36,7 @@ constexpr uint32_t kFusedEvents = 16384;    // most events of a level (a thread 
 constexpr uint32_t kFusedItems = 8192;      // most (state, rule) items of a level: one block scans them
 constexpr uint32_t kFusedLevels = 16;       // most levels of a launch (records in mapped memory)
 constexpr uint32_t kFusedEdges = 255;       // largest state record a level may produce
-constexpr uint32_t kFusedSlice = 32;        // most events a warp builds in one run
+constexpr uint32_t kFusedSlice = kListMax;  // most events a warp builds in one run
 static_assert(kFusedEvents <= kNumSMs * kFusedThreads, "one event per thread");
 constexpr uint32_t kRangeWords = 10;        // per level and evolution: see k_levels
 constexpr uint32_t kLevelWords = 8;         // per level: F, events, states, frontier, pairs, max ne / nocc
@@ -149,19 +149,11 @@ __device__ void fused_scan(uint32_t* a, uint32_t n, uint32_t* sh) {
 // Event a of the level against its later siblings [a + 1, end): kept events all (no cut here).
 // Returns the partners; writes them as (a, c) from out on when out is given.
 __device__ uint32_t fused_pairs(const DevPtrs& P, uint32_t a, uint32_t end, uint32_t in, uint2* out) {
-    const uint32_t na = P.rules[P.ev_rule[a]].n_lhs, ca0 = P.ev_coff[a];
     const unsigned long long ma = P.ev_bmask[a];
+    const bool exact = P.st_ne[in] <= 63;
     uint32_t n = 0;
     for (uint32_t c = a + 1; c < end && P.ev_in[c] == in; ++c) {
-        bool share = false;
-        if (ma) {
-            share = (ma & P.ev_bmask[c]) != 0ull;
-        } else {   // a parent of more than 63 edges: compare edge ids
-            const uint32_t nc = P.rules[P.ev_rule[c]].n_lhs, cc0 = P.ev_coff[c];
-            for (uint32_t k = 0; k < nc && !share; ++k)
-                for (uint32_t m = 0; m < na; ++m) share |= P.ev_cons[ca0 + m] == P.ev_cons[cc0 + k];
-        }
-        if (!share) continue;
+        if ((ma & P.ev_bmask[c]) == 0ull || !(exact || share_edge(P, a, c))) continue;
         if (out) out[n] = make_uint2(a, c);
         ++n;
     }
@@ -212,7 +204,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_levels(DevPtrs P, FusedArg
                     uint32_t cnt = 0;
                     if (r < ev.rule_count) {
                         load_rule(sm, L, &P.rules[ev.rule_begin + r]);
-                        if (pa.ne <= kLaneEMax && Rr.n_lhs <= kLaneJoinLhs) cnt = lane_join_count(L, sm, Rr, pa, vm);
+                        if (Rr.n_lhs <= kLaneJoinLhs) cnt = lane_join_count(L, sm, Rr, pa, vm);
                         else warp_join(L, sm, Rr, pa, Rr.sched, -1, [&](uint32_t) { ++cnt; }, 0xFFFFFFFFu,
                                        SkipCounter{&cnt, 0xFFFFFFFFu});
                     }
@@ -336,7 +328,6 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_levels(DevPtrs P, FusedArg
             uint32_t staged = kNone;
             Parent pa{0, 0, 0};
             bool pconn = false;
-            const unsigned long long* vm = nullptr;
             for (uint32_t t = lo_t, x = x0; x < x1; ++t) {
                 const uint32_t t0 = G.item_ev[t], rn = G.cnt[t];
                 if (x >= t0 + rn) continue;   // an item without events
@@ -346,9 +337,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_levels(DevPtrs P, FusedArg
                 if (f != staged) {
                     staged = f;
                     pa = load_parent(P, L, sm, sid);
-                    build_join_index(L, sm, pa);
                     pconn = parent_connected(L, sm, pa);
-                    vm = build_vmask(L, sm, pa);
                     if (lane == 0 && t0 == x) b_hbm += 4ull * (pa.ne + (pa.ne + 3) / 4 + pa.nocc) + 20;
                 }
                 load_rule(sm, L, &P.rules[ev.rule_begin + r]);
@@ -389,48 +378,15 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_levels(DevPtrs P, FusedArg
                     }
                     __syncwarp();
                 };
-                if (pa.ne <= kLaneEMax && Rr.n_lhs <= kLaneJoinLhs) {
-                    // lane walks: each lane counts its first edges' matches, the lanes holding the
-                    // run's matches list them (at most kFusedSlice), then one child after another
-                    uint32_t* list = smp<uint32_t>(sm, L.o_cand);   // the warp join's candidates: unused here
-                    const uint32_t cap = min(kFusedSlice, kMaxPatternEdges * L.W);
-                    for (uint32_t s0 = lo; s0 < hi; s0 += cap) {
-                        const uint32_t s1 = min(hi, s0 + cap);
-                        uint32_t done = 0;
-                        for (uint32_t e0b = 0; e0b < pa.ne; e0b += 32) {
-                            const uint32_t e0 = e0b + lane;
-                            const uint32_t c = e0 < pa.ne ? lane_walk(L, sm, Rr, pa, e0, vm, [](uint32_t) {}) : 0u;
-                            const uint32_t inc = warp_incl_scan(c);
-                            uint32_t at = done + inc - c;
-                            if (c && at < s1 && at + c > s0)
-                                lane_walk(L, sm, Rr, pa, e0, vm, [&](uint32_t pk) {
-                                    if (at >= s0 && at < s1) list[at - s0] = pk;
-                                    ++at;
-                                });
-                            done += __shfl_sync(0xFFFFFFFFu, inc, 31);
-                        }
-                        __syncwarp();
-                        if (done != rn) {
-                            if (lane == 0) atomicOr(P.err, kErrJoinCount);
-                            break;
-                        }
-                        for (uint32_t i = s0; i < s1; ++i) {
-                            const uint32_t pk = list[i - s0];
-                            uint16_t* pos = smp<uint16_t>(sm, L.o_mdepth);   // the warp join's scratch
-                            uint32_t* taken = smp<uint32_t>(sm, L.o_taken);
-                            __syncwarp();
-                            if (lane < Rr.n_lhs) pos[lane] = static_cast<uint16_t>((pk >> (8u * lane)) & 0xFFu);
-                            for (uint32_t k = lane; k < L.W; k += 32) taken[k] = 0;
-                            __syncwarp();
-                            fwd_emit(L, sm, Rr, pos, [&](uint32_t nm) { child(i, nm); });
-                        }
-                    }
-                } else {
-                    uint32_t idx = 0;
-                    warp_join(L, sm, Rr, pa, Rr.sched, -1, [&](uint32_t nm) {
-                        if (idx >= lo && idx < hi) child(idx, nm);
-                        ++idx;
-                    }, hi, SkipCounter{&idx, lo});
+                // the run's matches listed, then one child after another
+                const Fwd none{};
+                const uint16_t* mpos = smp<uint16_t>(sm, L.o_mpos);
+                uint32_t* taken = smp<uint32_t>(sm, L.o_taken);
+                if (list_matches(P, L, sm, Rr, pa, none, lo, hi, rn)) {
+                    for (uint32_t k = lane; k < L.W; k += 32) taken[k] = 0;
+                    __syncwarp();
+                    for (uint32_t i = lo; i < hi; ++i)
+                        fwd_emit(L, sm, Rr, mpos + (i - lo) * L.LH, [&](uint32_t nm) { child(i, nm); });
                 }
                 if (lane == 0 && lo == 0) b_stage += 4ull * pa.ne + 4ull * pa.nocc;
                 x = t0 + hi;

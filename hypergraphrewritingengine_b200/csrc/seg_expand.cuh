@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(256, 3) k_expand_seg(DevPtrs P, LevelArgs A, L
         bool conn;
         {   // packed edges, and whether the parent is one component
             uint32_t* pk_out = smp<uint32_t>(sm, L.o_ppk);
-            uint32_t* adj = smp<uint32_t>(sm, L.o_deg);   // load_parent's scratch
+            uint32_t* adj = smp<uint32_t>(sm, L.o_first);   // load_parent's scratch
             if (lane < pa.nvp) adj[lane] = 0;
             __syncwarp();
             for (uint32_t e = lane; e < pa.ne; e += 32) {

@@ -77,6 +77,12 @@ __device__ __forceinline__ void isort32(uint32_t* a, uint32_t n) {
     }
 }
 
+}  // namespace
+}  // namespace hgx
+#include "seg_wl.cuh"
+namespace hgx {
+namespace {
+
 // Warp-aggregated add of 1 to counter[key] for the lanes in `active`.
 __device__ __forceinline__ void warp_count(unsigned long long* counter, uint32_t key, bool active) {
     const uint32_t act = __ballot_sync(0xFFFFFFFFu, active);
@@ -176,8 +182,8 @@ __device__ Parent load_parent(const DevPtrs& P, const Layout& L, char* sm, uint3
     uint8_t* pear = smp<uint8_t>(sm, L.o_pear);
     uint16_t* pevo = smp<uint16_t>(sm, L.o_pevo);
     uint16_t* vloc = smp<uint16_t>(sm, L.o_vloc);
-    uint32_t* glob = smp<uint32_t>(sm, L.o_occ);    // aliases the WL occurrence list
-    uint32_t* first = smp<uint32_t>(sm, L.o_deg);   // aliases the WL degrees
+    uint32_t* glob = smp<uint32_t>(sm, L.o_glob);
+    uint32_t* first = smp<uint32_t>(sm, L.o_first);
     const uint32_t aw = (pa.ne + 3) >> 2;
     for (uint32_t i = lane; i < pa.ne; i += 32) {
         peid[i] = rec[i];
@@ -386,6 +392,18 @@ __device__ void build_join_index(const Layout& L, char* sm, const Parent& pa) {
         if (i <= pa.nvp) xoff[i] = i == 0 ? 0u : x;
         __syncwarp();
     }
+    // ascending edges in every list: a walk over it meets its candidates in canonical order
+    for (uint32_t v = lane; v < pa.nvp; v += 32) {
+        uint16_t* l = xinc + xoff[v];
+        const uint32_t m = xoff[v + 1] - xoff[v];
+        for (uint32_t i = 1; i < m; ++i) {
+            const uint16_t k = l[i];
+            uint32_t j = i;
+            while (j > 0 && l[j - 1] > k) { l[j] = l[j - 1]; --j; }
+            l[j] = k;
+        }
+    }
+    __syncwarp();
     // signature index: the distinct keys of each 32-edge chunk (match_any), appended to the
     // bucket list one leader at a time; more than kSigBuckets keys leaves it unbuilt
     for (uint32_t b = 0; b < pa.ne && misc[0] <= kSigBuckets; b += 32) {
@@ -806,12 +824,115 @@ __device__ const unsigned long long* build_vmask(const Layout& L, char* sm, cons
     return vm;
 }
 
+// The walk for states past 64 edges (positions of 16 bits, rules of at most kLaneJoinLhs edges): a
+// pattern edge with a bound variable is tried against the edges of the bound vertex of smallest
+// degree (the join index's ascending lists), else against every edge; on_match receives the
+// positions in pattern order, 16 bits each. Same matches in the same order as lane_walk.
+template <class F>
+__device__ uint32_t index_walk(const Layout& L, const char* csm, const DevRule& R, const Parent& pa,
+                               uint32_t e0, F&& on_match) {
+    char* sm = const_cast<char*>(csm);
+    const uint8_t* pear = smp<uint8_t>(sm, L.o_pear);
+    const uint16_t* pevo = smp<uint16_t>(sm, L.o_pevo);
+    const uint16_t* vloc = smp<uint16_t>(sm, L.o_vloc);
+    const bool indexed = L.XI && *smp<uint32_t>(sm, L.o_xready);
+    const uint32_t* xoff = smp<uint32_t>(sm, L.o_xoff);
+    const uint16_t* xinc = smp<uint16_t>(sm, L.o_xinc);
+    const uint32_t n = R.n_lhs;
+    uint16_t bind[kMaxVars];
+    uint32_t bound = 0;
+    uint32_t newly[kLaneJoinLhs], pick[kLaneJoinLhs], at[kLaneJoinLhs], end[kLaneJoinLhs];
+    auto try_bind = [&](uint32_t d, uint32_t j) -> bool {
+        const uint32_t p = R.sched[d], a = R.lhs_ar[p];
+        if (pear[j] != a) return false;
+        for (uint32_t k = 0; k < d; ++k)
+            if (pick[k] == j) return false;
+        const uint8_t* pv = &R.lhs_vars[R.lhs_off[p]];
+        const uint32_t vo = pevo[j];
+        uint32_t nb = 0;
+        for (uint32_t q = 0; q < a; ++q) {
+            const uint32_t var = pv[q];
+            const uint16_t x = vloc[vo + q];
+            if ((bound >> var) & 1u) {
+                if (bind[var] != x) { bound &= ~nb; return false; }
+            } else {
+                bind[var] = x;
+                bound |= 1u << var;
+                nb |= 1u << var;
+            }
+        }
+        newly[d] = nb;
+        pick[d] = j;
+        return true;
+    };
+    constexpr uint32_t kAll = 0x80000000u;   // at / end count edges, not list entries
+    auto enter = [&](uint32_t d) {
+        at[d] = kAll;
+        end[d] = kAll | pa.ne;
+        if (!indexed) return;
+        const uint32_t p = R.sched[d], a = R.lhs_ar[p];
+        const uint8_t* pv = &R.lhs_vars[R.lhs_off[p]];
+        uint32_t best = pa.ne + 1;
+        for (uint32_t q = 0; q < a; ++q) {
+            if (!((bound >> pv[q]) & 1u)) continue;
+            const uint32_t x = bind[pv[q]], deg = xoff[x + 1] - xoff[x];
+            if (deg < best) { best = deg; at[d] = xoff[x]; end[d] = xoff[x + 1]; }
+        }
+    };
+    if (!try_bind(0, e0)) return 0;
+    if (n == 1) {
+        on_match(static_cast<unsigned long long>(e0));
+        return 1;
+    }
+    uint32_t found = 0, d = 1;
+    enter(1);
+    while (true) {
+        bool ok = false;
+        while (at[d] != end[d]) {
+            const uint32_t j = (at[d] & kAll) ? at[d] & ~kAll : xinc[at[d]];
+            ++at[d];
+            if (try_bind(d, j)) { ok = true; break; }
+        }
+        if (ok) {
+            if (d + 1 == n) {
+                unsigned long long packed = 0;
+                for (uint32_t k = 0; k < n; ++k) packed |= static_cast<unsigned long long>(pick[k]) << (16u * R.sched[k]);
+                on_match(packed);
+                ++found;
+                bound &= ~newly[d];
+            } else {
+                ++d;
+                enter(d);
+            }
+        } else {
+            --d;
+            if (d == 0) break;
+            bound &= ~newly[d];
+        }
+    }
+    return found;
+}
+
+// States whose match counts are kept per 32 first edges (LevelArgs::chunks).
+__device__ __forceinline__ bool chunked(uint32_t ne) { return ne > kLaneEMax && ne <= 32 * kChunks; }
+
 // Matches of (state, rule) by lane walks over every first edge, warp total. A state of at most 16
 // (8) edges gives each first edge 2 (4) lanes, which split the second position's candidates.
 __device__ uint32_t lane_join_count(const Layout& L, const char* sm, const DevRule& R,
-                                    const Parent& pa, const unsigned long long* vm) {
+                                    const Parent& pa, const unsigned long long* vm,
+                                    uint32_t* chunks = nullptr, uint32_t part = 0,
+                                    uint32_t n_parts = 1) {
     uint32_t c = 0;
     const uint32_t lane = lane_id();
+    if (chunks && chunked(pa.ne)) {
+        // a large state: this warp's groups of 32 first edges, with the matches of each kept
+        for (uint32_t b = 32 * part; b < pa.ne; b += 32 * n_parts) {
+            const uint32_t n = warp_sum32(b + lane < pa.ne ? index_walk(L, sm, R, pa, b + lane, [](unsigned long long) {}) : 0u);
+            if (lane == 0) chunks[b >> 5] = n;
+            c += n;
+        }
+        return c;
+    }
     const uint32_t parts = (R.n_lhs < 2 || pa.ne > 16) ? 1u : (pa.ne <= 8 ? 4u : 2u);
     if (parts > 1) {
         const uint32_t e0 = lane / parts, part = lane % parts;
@@ -820,8 +941,11 @@ __device__ uint32_t lane_join_count(const Layout& L, const char* sm, const DevRu
             c = lane_walk(L, sm, R, pa, e0, vm, [](uint32_t) {}, part * span, (part + 1) * span);
         return warp_sum32(c);
     }
-    for (uint32_t b = 0; b < pa.ne; b += 32)
-        if (b + lane < pa.ne) c += lane_walk(L, sm, R, pa, b + lane, vm, [](uint32_t) {});
+    for (uint32_t b = 0; b < pa.ne; b += 32) {
+        if (b + lane >= pa.ne) continue;
+        if (pa.ne <= kLaneEMax) c += lane_walk(L, sm, R, pa, b + lane, vm, [](uint32_t) {});
+        else c += index_walk(L, sm, R, pa, b + lane, [](unsigned long long) {});
+    }
     return warp_sum32(c);
 }
 
@@ -951,8 +1075,60 @@ __device__ bool parent_connected(const Layout& L, char* sm, const Parent& pa) {
     return one;
 }
 
+// FNV fold, in ascending order, of one vertex's neighbour words when they do not fit the buffer: the
+// warp finds the smallest word above the last one and how often it occurs, until all are folded.
+__device__ uint64_t fold_oversize(const uint8_t* car, const uint16_t* cvo, const uint16_t* vloc,
+                                  const uint16_t* o, uint32_t dv, uint32_t left, const uint64_t* cur, uint64_t h) {
+    const uint32_t lane = lane_id();
+    uint64_t last = 0;
+    bool any = false;
+    while (left) {
+        uint64_t m = ~0ull;
+        uint32_t c = 0;
+        for (uint32_t j = lane; j < dv; j += 32) {
+            const uint32_t e = o[j] >> 4, q = o[j] & 15u, a = car[e], vo = cvo[e];
+            for (uint32_t k = 0; k < a; ++k) {
+                if (k == q) continue;
+                const uint64_t x = fnv(cur[vloc[vo + k]], k);
+                if (any && x <= last) continue;
+                if (x < m) { m = x; c = 1; }
+                else if (x == m) ++c;
+            }
+        }
+        uint64_t least = m;
+#pragma unroll
+        for (int d = 16; d; d >>= 1) {
+            const uint64_t y = __shfl_xor_sync(0xFFFFFFFFu, least, d);
+            least = y < least ? y : least;
+        }
+        const uint32_t n = warp_sum32(m == least ? c : 0u);
+        if (!n) break;   // (every word is folded: left counts them)
+        for (uint32_t k = 0; k < n; ++k) h = fnv(h, least);
+        last = least;
+        any = true;
+        left -= min(left, n);
+    }
+    return h;
+}
+
+// The sorted fold of a lane's n words at l, shortest network that takes the warp's longest list.
+__device__ __forceinline__ uint64_t fold_any(uint64_t* l, uint32_t n, uint32_t n_max, uint64_t h) {
+    if (n_max <= 8) return fold_sorted<8>(l, n, n_max, h);
+    if (n_max <= 16) return fold_sorted<16>(l, n, n_max, h);
+    if (n_max <= 32) return fold_sorted<32>(l, n, n_max, h);
+    return fold_exact(l, n, h);
+}
+
 // connected: the child is known to be one component (a connected parent under a rule whose
 // right-hand side joins every left-hand vertex): the union-find is skipped.
+//
+// Lanes take vertices in groups: as many consecutive ones, at most 32, as have their neighbour words
+// fit the buffer. States of 260 ternary edges need 16 KB of shared memory a warp (37 KB when the
+// buffer held every vertex's words and the distinct-colour set, the component sums and the join's
+// structures had bytes of their own): 12 warps an SM in place of 5. With sorting in registers, matches
+// listed a group of first edges at a time and smaller units on small launches the warp kernel takes
+// 18.6 ms in place of 27.9 over 129 evolutions of 65-256-edge states, 16.4 in place of 30 over the
+// 1,024 random evolutions.
 __device__ uint64_t warp_wl(const Layout& L, char* sm, uint32_t ne, uint32_t V, WlInfo& info,
                         bool connected = false) {
     const uint32_t lane = lane_id();
@@ -961,12 +1137,9 @@ __device__ uint64_t warp_wl(const Layout& L, char* sm, uint32_t ne, uint32_t V, 
     const uint16_t* vloc = smp<uint16_t>(sm, L.o_vloc);
     uint64_t* cur = smp<uint64_t>(sm, L.o_cur);
     uint64_t* nxt = smp<uint64_t>(sm, L.o_nxt);
-    uint64_t* csum = smp<uint64_t>(sm, L.o_csum);
-    uint64_t* ccnt = smp<uint64_t>(sm, L.o_ccnt);
-    uint64_t* nbr = smp<uint64_t>(sm, L.o_nbr);
-    uint32_t* occ = smp<uint32_t>(sm, L.o_occ);
+    uint64_t* buf = smp<uint64_t>(sm, L.o_buf);
+    uint16_t* occ = smp<uint16_t>(sm, L.o_occ);
     uint32_t* ooff = smp<uint32_t>(sm, L.o_ooff);
-    uint32_t* nbo = smp<uint32_t>(sm, L.o_nbo);
     uint32_t* deg = smp<uint32_t>(sm, L.o_deg);
     uint32_t* nn = smp<uint32_t>(sm, L.o_nn);
     uint32_t* comp = smp<uint32_t>(sm, L.o_comp);
@@ -977,102 +1150,165 @@ __device__ uint64_t warp_wl(const Layout& L, char* sm, uint32_t ne, uint32_t V, 
     info.nbr = 0;
     if (ne == 0) return kEmptyStateHash;
 
-    for (uint32_t v = lane; v < V; v += 32) { deg[v] = 0; nn[v] = 0; }
+    // degrees and neighbour counts; comp: occurrences by position, a byte each (one arity of 2..4)
+    for (uint32_t v = lane; v < V; v += 32) { deg[v] = 0; nn[v] = 0; comp[v] = 0; }
     __syncwarp();
+    const uint32_t a0 = car[0];
+    bool uni = a0 >= 2 && a0 <= 4;
     for (uint32_t e = lane; e < ne; e += 32) {
         const uint32_t a = car[e], vo = cvo[e];
+        uni = uni && a == a0;
         for (uint32_t q = 0; q < a; ++q) {
             const uint32_t v = vloc[vo + q];
             atomicAdd(&deg[v], 1u);
             atomicAdd(&nn[v], a - 1u);
+            if (q < 4) atomicAdd(&comp[v], 1u << (8 * q));
         }
     }
+    uni = __all_sync(0xFFFFFFFFu, uni);
     __syncwarp();
-    uint32_t run_o = 0, run_n = 0, run_nn = 0, nv = 0, cap = 1;
+    uint32_t run_o = 0, run_nn = 0, nv = 0, cap = 1, dmax = 0;
     for (uint32_t b = 0; b < V; b += 32) {
         const uint32_t v = b + lane;
         const uint32_t dv = v < V ? deg[v] : 0u;
         const uint32_t nnv = v < V ? nn[v] : 0u;
-        const uint32_t s = max(nnv, dv);
         const uint32_t io = warp_incl_scan(dv);
-        const uint32_t is = warp_incl_scan(s);
-        if (v < V) {
-            ooff[v] = run_o + io - dv;
-            nbo[v] = run_n + is - s;
-            comp[v] = run_o + io - dv;
-        }
+        if (v < V) ooff[v] = run_o + io - dv;
         run_o += __shfl_sync(0xFFFFFFFFu, io, 31);
-        run_n += __shfl_sync(0xFFFFFFFFu, is, 31);
         nv += __popc(__ballot_sync(0xFFFFFFFFu, dv > 0));
         cap = max(cap, warp_max32(nnv));
+        dmax = max(dmax, warp_max32(dv));
         run_nn += warp_sum32(nnv);
     }
     info.nv = nv;
     info.nocc = run_o;
     info.nbr = run_nn;   // sum over edges of a(a-1): neighbour entries per refinement round
     if (nv == 0) return 0;   // only arity-0 edges: the reference core returns 0
+    const bool counted = uni && dmax < 256;
+    // initial colours of a single arity: the positions in order with their multiplicities
+    if (counted)
+        for (uint32_t v = lane; v < V; v += 32) {
+            const uint32_t c = comp[v];
+            uint64_t h = fnv(kFnvOffset, static_cast<uint64_t>(deg[v]));
+            for (uint32_t q = 0; q < a0; ++q)
+                for (uint32_t j = (c >> (8 * q)) & 0xFFu; j; --j) h = fnv(fnv(h, a0), q);
+            cur[v] = h;
+        }
+    __syncwarp();
+    for (uint32_t v = lane; v < V; v += 32) comp[v] = ooff[v];
     __syncwarp();
     for (uint32_t e = lane; e < ne; e += 32) {
         const uint32_t a = car[e], vo = cvo[e];
         for (uint32_t q = 0; q < a; ++q) {
             const uint32_t slot = atomicAdd(&comp[vloc[vo + q]], 1u);
-            occ[slot] = (e << 8) | q;
+            occ[slot] = static_cast<uint16_t>((e << 4) | q);
         }
     }
     __syncwarp();
 
-    // initial colours
-    for (uint32_t v = lane; v < V; v += 32) {
-        const uint32_t dv = deg[v];
-        if (!dv) continue;
-        uint32_t* o = occ + ooff[v];
-        if (dv > cap) isort32(o, dv);   // truncation keeps the first `cap` in edge order
-        uint64_t* kb = nbr + nbo[v];
-        const uint32_t n = min(dv, cap);
-        for (uint32_t j = 0; j < n; ++j) {
-            const uint32_t x = o[j];
-            kb[j] = (static_cast<uint64_t>(car[x >> 8]) << 8) | (x & 0xFFu);
+    // groups of consecutive vertices whose words fit the buffer: on_group(v, n, base, n_max) on the
+    // lanes of the group (n 0 on the others), on_big(v, n) where one vertex alone does not fit
+    auto groups = [&](auto&& count, auto&& on_group, auto&& on_big) {
+        for (uint32_t v0 = 0; v0 < V;) {
+            const uint32_t v = v0 + lane;
+            uint32_t n = v < V ? count(v) : 0u;
+            const uint32_t inc = warp_incl_scan(n);
+            const uint32_t fit = __ballot_sync(0xFFFFFFFFu, v < V && inc <= L.BUF);
+            const uint32_t take = __popc(fit);   // (a prefix of the lanes: inc does not fall)
+            if (!take) {
+                on_big(v0, __shfl_sync(0xFFFFFFFFu, n, 0));
+                ++v0;
+                continue;
+            }
+            if (lane >= take) n = 0;
+            on_group(v, n, inc - n, warp_max32(n), lane < take);
+            __syncwarp();
+            v0 += take;
         }
-        isort64(kb, n);
-        uint64_t h = fnv(kFnvOffset, static_cast<uint64_t>(dv));
-        for (uint32_t j = 0; j < n; ++j) {
-            h = fnv(h, kb[j] >> 8);
-            h = fnv(h, kb[j] & 0xFFu);
-        }
-        cur[v] = h;
+    };
+    if (!counted) {
+        // initial colours: sorted (arity, position) of the first `cap` occurrences in edge order
+        groups([&](uint32_t v) { return min(deg[v], cap); },
+               [&](uint32_t v, uint32_t n, uint32_t base, uint32_t, bool mine) {
+            if (!mine || !deg[v]) return;
+            uint16_t* o = occ + ooff[v];
+            const uint32_t dv = deg[v];
+            if (dv > cap)   // truncation keeps the first `cap` in edge order
+                for (uint32_t i = 1; i < dv; ++i) {
+                    const uint16_t k = o[i];
+                    uint32_t j = i;
+                    while (j > 0 && o[j - 1] > k) { o[j] = o[j - 1]; --j; }
+                    o[j] = k;
+                }
+            uint64_t* kb = buf + base;
+            for (uint32_t j = 0; j < n; ++j) kb[j] = (static_cast<uint64_t>(car[o[j] >> 4]) << 8) | (o[j] & 15u);
+            isort64(kb, n);
+            uint64_t h = fnv(kFnvOffset, static_cast<uint64_t>(dv));
+            for (uint32_t j = 0; j < n; ++j) {
+                h = fnv(h, kb[j] >> 8);
+                h = fnv(h, kb[j] & 0xFFu);
+            }
+            cur[v] = h;
+        }, [&](uint32_t v, uint32_t n) {
+            // one vertex of more occurrences than the buffer: a counting pass per (arity, position)
+            uint16_t* o = occ + ooff[v];
+            const uint32_t dv = deg[v];
+            if (dv > cap && lane == 0)
+                for (uint32_t i = 1; i < dv; ++i) {
+                    const uint16_t k = o[i];
+                    uint32_t j = i;
+                    while (j > 0 && o[j - 1] > k) { o[j] = o[j - 1]; --j; }
+                    o[j] = k;
+                }
+            __syncwarp();
+            uint64_t h = fnv(kFnvOffset, static_cast<uint64_t>(dv));
+            for (uint32_t a = 1; a <= static_cast<uint32_t>(kMaxArity); ++a)
+                for (uint32_t q = 0; q < a; ++q) {
+                    uint32_t c = 0;
+                    for (uint32_t j = lane; j < n; j += 32) c += car[o[j] >> 4] == a && (o[j] & 15u) == q ? 1u : 0u;
+                    c = warp_sum32(c);
+                    for (uint32_t j = 0; j < c; ++j) h = fnv(fnv(h, a), q);
+                }
+            if (lane == 0) cur[v] = h;
+            __syncwarp();
+        });
     }
     __syncwarp();
-    uint64_t* srt = smp<uint64_t>(sm, L.o_srt);
-    uint32_t prev = wl_distinct(cur, deg, V, nv, srt);
+    uint32_t prev = wl_distinct(cur, deg, V, nv, buf);
     for (uint32_t it = 0; it < kWlMaxRounds; ++it) {
-        for (uint32_t v = lane; v < V; v += 32) {
-            const uint32_t dv = deg[v];
-            if (!dv) continue;
-            const uint32_t* o = occ + ooff[v];
-            uint64_t* kb = nbr + nbo[v];
-            uint32_t n = 0;
-            for (uint32_t j = 0; j < dv; ++j) {
-                const uint32_t x = o[j];
-                const uint32_t e = x >> 8, q = x & 0xFFu;
-                const uint32_t a = car[e], vo = cvo[e];
-                for (uint32_t k = 0; k < a; ++k)
-                    if (k != q && n < cap) kb[n++] = fnv(cur[vloc[vo + k]], k);
+        // (nn[v] <= cap, so the reference's cap never cuts a neighbour list)
+        groups([&](uint32_t v) { return nn[v]; },
+               [&](uint32_t v, uint32_t n, uint32_t base, uint32_t n_max, bool mine) {
+            uint64_t* kb = buf + base;
+            if (mine && deg[v]) {
+                const uint16_t* o = occ + ooff[v];
+                uint32_t m = 0;
+                for (uint32_t j = 0, dv = deg[v]; j < dv; ++j) {
+                    const uint32_t e = o[j] >> 4, q = o[j] & 15u, a = car[e], vo = cvo[e];
+                    for (uint32_t k = 0; k < a; ++k)
+                        if (k != q) kb[m++] = fnv(cur[vloc[vo + k]], k);
+                }
             }
-            isort64(kb, n);
-            uint64_t h = cur[v];
-            for (uint32_t j = 0; j < n; ++j) h = fnv(h, kb[j]);
-            nxt[v] = h;
-        }
+            const uint64_t h = fold_any(kb, n, n_max, mine ? cur[v] : 0ull);
+            if (mine && deg[v]) nxt[v] = h;
+        }, [&](uint32_t v, uint32_t n) {
+            const uint64_t h = fold_oversize(car, cvo, vloc, occ + ooff[v], deg[v], n, cur, cur[v]);
+            if (lane == 0) nxt[v] = h;
+            __syncwarp();
+        });
+        uint64_t* t = cur;
+        cur = nxt;
+        nxt = t;
         __syncwarp();
-        for (uint32_t v = lane; v < V; v += 32) cur[v] = nxt[v];
-        __syncwarp();
-        const uint32_t dd = wl_distinct(cur, deg, V, nv, srt);
+        const uint32_t dd = wl_distinct(cur, deg, V, nv, buf);
         ++info.rounds;
         if (dd == prev) break;
         prev = dd;
     }
 
-    // components (union-find on one lane; the partition is what enters the hash)
+    // components (union-find over the edges; the partition is what enters the hash)
+    uint64_t* csum = buf;
+    uint64_t* ccnt = buf + V;
     bool one = connected;
     if (!connected) {
         for (uint32_t v = lane; v < V; v += 32) { comp[v] = v; csum[v] = 0; ccnt[v] = 0; }
@@ -1351,6 +1587,70 @@ __device__ void enumerate_matches(const DevPtrs& P, const Layout& L, char* sm, c
     while (j < f.nd) fwd_emit(L, sm, R, dpos2 + j++ * kFwdMaxLhs, on_match);
 }
 
+// State positions (pattern order, L.LH apart) of the staged state's matches [lo, hi), at most
+// kListMax of them, into the layout's list; rn: the matches the count pass found. The join's
+// structures may be overwritten once this returns (they share their bytes with the WL arrays).
+// False (and an error flag) when the join finds another number of matches.
+__device__ bool list_matches(const DevPtrs& P, const Layout& L, char* sm, const DevRule& R, const Parent& pa,
+                             const Fwd& f, uint32_t lo, uint32_t hi, uint32_t rn,
+                             const uint32_t* chunks = nullptr) {
+    const uint32_t lane = lane_id(), n_lhs = R.n_lhs;
+    uint16_t* mpos = smp<uint16_t>(sm, L.o_mpos);
+    if (!f.on && n_lhs <= kLaneJoinLhs) {
+        const bool small = pa.ne <= kLaneEMax;
+        const unsigned long long* vm = nullptr;
+        if (small) vm = build_vmask(L, sm, pa);
+        else build_join_index(L, sm, pa);
+        // where the count pass kept the matches before every 32 first edges: only the first edges of
+        // this run are walked (of a 256-edge state one or two groups of eight)
+        uint32_t total = 0, b0 = 0;
+        const bool skip = chunks && chunked(pa.ne);
+        if (skip) {
+            const uint32_t n = (pa.ne + 31) >> 5, mine = lane < n ? chunks[lane] : 0u;
+            const uint32_t before = warp_incl_scan(mine) - mine;
+            b0 = 32 * (__popc(__ballot_sync(0xFFFFFFFFu, lane < n && before <= lo)) - 1);
+            total = __shfl_sync(0xFFFFFFFFu, before, b0 >> 5);
+        }
+        for (uint32_t b = b0; b < pa.ne && !(skip && total >= hi); b += 32) {
+            const uint32_t e0 = b + lane;
+            uint32_t c = 0;
+            if (e0 < pa.ne)
+                c = small ? lane_walk(L, sm, R, pa, e0, vm, [](uint32_t) {})
+                          : index_walk(L, sm, R, pa, e0, [](unsigned long long) {});
+            const uint32_t inc = warp_incl_scan(c);
+            uint32_t at = total + inc - c;
+            if (c && at < hi && at + c > lo) {
+                auto put = [&](unsigned long long pk, uint32_t bits) {
+                    if (at >= lo && at < hi)
+                        for (uint32_t k = 0; k < n_lhs; ++k)
+                            mpos[(at - lo) * L.LH + k] = static_cast<uint16_t>((pk >> (bits * k)) & ((1u << bits) - 1u));
+                    ++at;
+                };
+                if (small) lane_walk(L, sm, R, pa, e0, vm, [&](uint32_t pk) { put(pk, 8); });
+                else index_walk(L, sm, R, pa, e0, [&](unsigned long long pk) { put(pk, 16); });
+            }
+            total += __shfl_sync(0xFFFFFFFFu, inc, 31);
+        }
+        __syncwarp();
+        if (skip ? total < hi : total != rn) {
+            if (lane == 0) atomicOr(P.err, kErrJoinCount);
+            return false;
+        }
+        return true;
+    }
+    if (!f.on) build_join_index(L, sm, pa);
+    const uint16_t* match = smp<uint16_t>(sm, L.o_match);
+    uint32_t idx = 0;
+    // matches before the run are skipped whole at the last position (popcounts)
+    enumerate_matches(P, L, sm, R, pa, f, [&](uint32_t) {
+        if (idx >= lo && idx < hi)
+            for (uint32_t k = lane; k < n_lhs; k += 32) mpos[(idx - lo) * L.LH + k] = match[k];
+        ++idx;
+    }, hi, SkipCounter{&idx, lo});
+    __syncwarp();
+    return true;
+}
+
 // Number of matches under forwarding (F survivors + D).
 __device__ uint32_t fwd_count(const DevPtrs& P, const Layout& L, char* sm, const DevRule& R,
                               const Parent& pa, const Fwd& f) {
@@ -1549,12 +1849,15 @@ __global__ void __launch_bounds__(256, 4) k_count(DevPtrs P, LevelArgs A, Layout
     char* sm = smem + (threadIdx.x >> 5) * L.bytes;
     const uint32_t lane = lane_id();
     const DevRule& R = *smp<DevRule>(sm, L.o_rule);
-    uint32_t max_cnt = 0;   // largest match count of a (state, rule) this warp counted
+    const uint32_t n_parts = A.parts;   // warps per large state (1: none is split)
     WarpWork q;
     while (true) {
-        const uint32_t f = q.next(&A.work[0]);
+        const uint32_t u = q.next(&A.work[0]);
+        const uint32_t f = u / n_parts, part = u - f * n_parts;
         if (f >= A.n_frontier) break;
         const uint32_t sid = A.frontier[f];
+        const bool split = n_parts > 1 && chunked(P.st_ne[sid]);
+        if (part && !split) continue;
         const Parent pa = load_parent(P, L, sm, sid);
         build_join_index(L, sm, pa);
         const unsigned long long* vm = build_vmask(L, sm, pa);
@@ -1584,30 +1887,37 @@ __global__ void __launch_bounds__(256, 4) k_count(DevPtrs P, LevelArgs A, Layout
                 lane_ok = lane_ok && pa.nvp + R.n_fresh <= A.lane_vmax && pnn_max + gain <= kLaneNMax;
                 seg_ok = seg_ok && pa.nvp + R.n_fresh <= static_cast<uint32_t>(kLaneVMax) &&
                          pa.ne + R.n_rhs <= kSegEMax + R.n_lhs;
+                if (part && R.n_lhs > kLaneJoinLhs) continue;   // counted whole by part 0
                 const Fwd fw = fwd_prepare(P, A, L, sm, R, ev, pa, sid, true);
                 fwd_on = fw.on;
                 if (fw.on) cnt = fwd_count(P, L, sm, R, pa, fw);
-                else if (pa.ne <= kLaneEMax && R.n_lhs <= kLaneJoinLhs) cnt = lane_join_count(L, sm, R, pa, vm);
+                else if (R.n_lhs <= kLaneJoinLhs)
+                    cnt = lane_join_count(L, sm, R, pa, vm,
+                                          A.chunks ? A.chunks + (uint64_t(f) * A.rules_stride + r) * kChunks : nullptr,
+                                          split ? part : 0u, split ? n_parts : 1u);
                 else warp_join(L, sm, R, pa, R.sched, -1, [&](uint32_t) { ++cnt; }, 0xFFFFFFFFu,
                                SkipCounter{&cnt, 0xFFFFFFFFu});
             }
-            if (lane == 0) A.counts[f * A.rules_stride + r] = cnt;
-            max_cnt = max(max_cnt, cnt);
+            if (lane == 0) {
+                if (split) atomicAdd(&A.counts[f * A.rules_stride + r], cnt);   // (zeroed before)
+                else A.counts[f * A.rules_stride + r] = cnt;
+            }
             __syncwarp();
         }
-        if (lane == 0) A.fmode[f] = (lane_ok ? 1 : 0) | (fwd_on ? 2 : 0) | (seg_ok ? 4 : 0);
+        if (lane == 0 && part == 0) A.fmode[f] = (lane_ok ? 1 : 0) | (fwd_on ? 2 : 0) | (seg_ok ? 4 : 0);
     }
-    if (lane == 0 && max_cnt) atomicMax(&A.level_max[4], max_cnt);   // sizes the staged match list
 }
 
 // Per-item counts scaled by the rule's consumed / produced / fresh sizes, for the scans.
 __global__ void k_item_sizes(DevPtrs P, LevelArgs A) {
     const uint32_t n = A.n_frontier * A.rules_stride;
+    uint32_t max_cnt = 0;   // largest match count of a (state, rule): sizes the staged match list
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
         const uint32_t f = t / A.rules_stride, r = t % A.rules_stride;
         const uint32_t sid = A.frontier[f];
         const DevEvo& ev = P.evos[P.st_evo[sid]];
         const uint32_t c = A.counts[t];
+        max_cnt = max(max_cnt, c);
         uint32_t cons = 0, prod = 0, fresh = 0;
         if (r < ev.rule_count && c) {
             const DevRule& R = P.rules[ev.rule_begin + r];
@@ -1620,19 +1930,33 @@ __global__ void k_item_sizes(DevPtrs P, LevelArgs A) {
         A.item_prod[t] = prod;
         A.item_fresh[t] = fresh;
     }
+    max_cnt = warp_max32(max_cnt);
+    if (lane_id() == 0 && max_cnt) atomicMax(&A.level_max[4], max_cnt);
 }
 
 // An event's consumed parent positions as a bit mask for the branchial test (events of one input
-// state share the parent's positions, so equal positions are equal edges), or 0 when the parent
-// has more than 63 edges (the test then compares edge ids). Bit 63 is never a position: an event
-// that is not kept carries kMaskDropped, which shares no position with any other mask.
+// state share the parent's positions, so equal positions are equal edges). Exact for parents of at
+// most 63 edges; for larger ones bit p % 63 stands for position p, and a common bit only says that
+// the edge ids have to be compared. Bit 63 is never a position: an event that is not kept carries
+// kMaskDropped, which has no bit in common with any other mask.
 constexpr unsigned long long kMaskDropped = 1ull << 63;
 
 __device__ __forceinline__ unsigned long long branch_mask(uint32_t n, uint32_t pne, const uint8_t* pos) {
-    if (pne > 63) return 0ull;
     unsigned long long m = 0;
-    for (uint32_t k = 0; k < n; ++k) m |= 1ull << pos[k];
+    for (uint32_t k = 0; k < n; ++k) m |= 1ull << (pne > 63 ? pos[k] % 63u : pos[k]);
     return m;
+}
+
+// Whether two events consumed a common edge, by edge ids.
+__device__ bool share_edge(const DevPtrs& P, uint32_t a, uint32_t c) {
+    const uint32_t na = P.rules[P.ev_rule[a]].n_lhs, ca = P.ev_coff[a];
+    const uint32_t nc = P.rules[P.ev_rule[c]].n_lhs, cc = P.ev_coff[c];
+    bool share = false;
+    for (uint32_t k = 0; k < nc && !share; ++k) {
+        const uint32_t x = P.ev_cons[cc + k];
+        for (uint32_t m = 0; m < na; ++m) share |= P.ev_cons[ca + m] == x;
+    }
+    return share;
 }
 
 // Frontier position of work index w (identity unless the level runs over a list of ranges).
@@ -1647,15 +1971,6 @@ __device__ __forceinline__ uint32_t frontier_at(const LevelArgs& A, uint32_t w) 
     return A.frng[a] + (w - off[a]);
 }
 
-// Children per slice of a parent hashed warp-per-child: the smallest power of two >= 4 and
-// >= sqrt(children), so a parent with many children is spread over about sqrt(children) warps
-// while each warp re-enumerates at most its slice's end of the parent's matches.
-__device__ __forceinline__ uint32_t slice_size(uint32_t children) {
-    uint32_t s = 4;
-    while (uint64_t(s) * s < children) s <<= 1;
-    return s;
-}
-
 __device__ __forceinline__ uint32_t children_of(const LevelArgs& A, uint32_t f) {
     return A.item_ev[(f + 1) * A.rules_stride] - A.item_ev[f * A.rules_stride];
 }
@@ -1665,7 +1980,7 @@ __global__ void k_slice_counts(LevelArgs A, uint32_t n, uint32_t* cnt) {
     for (uint32_t w = blockIdx.x * blockDim.x + threadIdx.x; w < n; w += gridDim.x * blockDim.x) {
         const uint32_t f = frontier_at(A, A.f_begin + w);
         const uint32_t c = children_of(A, f);
-        cnt[w] = ((A.fmode[f] & A.path) || !c) ? 0u : (c + slice_size(c) - 1) / slice_size(c);
+        cnt[w] = (A.fmode[f] & A.path) ? 0u : (c + A.wslice - 1) / A.wslice;
     }
 }
 
@@ -1704,9 +2019,8 @@ __global__ void __launch_bounds__(256, 3) k_expand(DevPtrs P, LevelArgs A, Layou
                 if (A.soff[m] <= u) a = m; else b = m;
             }
             f = frontier_at(A, A.f_begin + a);
-            const uint32_t S = slice_size(children_of(A, f));
-            c_lo = (u - A.soff[a]) * S;
-            c_hi = c_lo + S;
+            c_lo = (u - A.soff[a]) * A.wslice;
+            c_hi = c_lo + A.wslice;
         }
         const uint8_t fm = A.fmode[f];
         if (((fm & A.path) != 0) != kLane) continue;
@@ -1716,7 +2030,6 @@ __global__ void __launch_bounds__(256, 3) k_expand(DevPtrs P, LevelArgs A, Layou
         const DevEvo ev = P.evos[evo];
         if (lane == 0 && c_lo == 0) b_hbm += 4ull * (pa.ne + (pa.ne + 3) / 4 + pa.nocc) + 20;
         if (kLane) build_parent_csr(L, sm, pa);
-        else build_join_index(L, sm, pa);
         // warp path: whether the parent is one component (then so is every child of a rule whose
         // right-hand side joins its left-hand vertices, and warp_wl skips its union-find)
         const bool pconn = !kLane && parent_connected(L, sm, pa);
@@ -1732,6 +2045,7 @@ __global__ void __launch_bounds__(256, 3) k_expand(DevPtrs P, LevelArgs A, Layou
             const uint32_t prod0 = A.prod_base + A.item_prod[item];
             const uint32_t fresh0 = A.fresh_base + A.item_fresh[item];
             const uint32_t rule_g = ev.rule_begin + r;
+            if (!kLane && (fm & 2u)) build_join_index(L, sm, pa);   // for the seeded joins
             const Fwd fwd = fwd_prepare(P, A, L, sm, R, ev, pa, sid, (fm & 2u) != 0);
             // per-child work shared by both paths: the event record and the table insert
             auto finish = [&](uint32_t idx, uint64_t h, const WlInfo& info, const uint8_t* rpos) {
@@ -1838,14 +2152,19 @@ __global__ void __launch_bounds__(256, 3) k_expand(DevPtrs P, LevelArgs A, Layou
                 if (nb) flush();
               }
             } else {
-                // this rule's children inside the unit's slice: [lo, hi) of its match order
+                // this rule's children inside the unit's slice: [lo, hi) of its match order, listed,
+                // then built and hashed one after another
                 const uint32_t lo = c_lo > rb ? c_lo - rb : 0u;
                 const uint32_t hi = min(rn, c_hi - rb);
-                uint32_t idx = 0;
+                if (!list_matches(P, L, sm, R, pa, fwd, lo, hi, rn,
+                                  A.chunks ? A.chunks + uint64_t(item) * kChunks : nullptr)) continue;
+                const uint16_t* mpos = smp<uint16_t>(sm, L.o_mpos);
+                uint32_t* taken = smp<uint32_t>(sm, L.o_taken);
+                for (uint32_t k = lane; k < L.W; k += 32) taken[k] = 0;
+                __syncwarp();
                 uint8_t rpos[kMaxPatternEdges];
-                // matches before the slice are skipped whole at the last position (popcounts)
-                enumerate_matches(P, L, sm, R, pa, fwd, [&](uint32_t nm) {
-                    if (idx >= lo && idx < hi) {
+                for (uint32_t idx = lo; idx < hi; ++idx)
+                    fwd_emit(L, sm, R, mpos + (idx - lo) * L.LH, [&](uint32_t nm) {
                         for (uint32_t k = 0; k < R.n_lhs; ++k) rpos[k] = static_cast<uint8_t>(match[k]);
                         const uint32_t nec = build_child(L, sm, R, pa, nm);
                         WlInfo info;
@@ -1853,9 +2172,7 @@ __global__ void __launch_bounds__(256, 3) k_expand(DevPtrs P, LevelArgs A, Layou
                                                    pconn && (R.flags & kRuleRhsJoinsLhs));
                         if (lane == 0) finish(idx, h, info, rpos);
                         __syncwarp();
-                    }
-                    ++idx;
-                }, hi, SkipCounter{&idx, lo});
+                    });
             }
         }
     }
@@ -2274,7 +2591,6 @@ __global__ void __launch_bounds__(256, kWalk ? 4 : 3) k_expand_lanes2(DevPtrs P,
 }
 
 }  // namespace hgx
-#include "seg_wl.cuh"
 #include "seg_expand.cuh"
 namespace hgx {
 
@@ -2605,7 +2921,7 @@ __global__ void k_rep(DevPtrs P, LevelArgs A) {
             rep = kept && (ev.quotient ? fresh : true);
             const bool front = rep && (P.st_depth[sid] + 1 < ev.steps) && cut == kNone;
             P.ev_kept[e] = kept ? 1 : 0;
-            if (!kept && P.ev_bmask[e]) P.ev_bmask[e] = kMaskDropped;
+            if (!kept) P.ev_bmask[e] = kMaskDropped;
             A.flag_rep[t] = rep ? 1u : 0u;
             A.flag_front[t] = front ? 1u : 0u;
             if (e == cut) P.evo_stopped[evo] = 1;
@@ -2871,56 +3187,31 @@ __global__ void __launch_bounds__(256, 4) k_materialize(DevPtrs P, LevelArgs A, 
 // order). Pass 0 counts a's pairs into bcount[t]; pass 1 writes them at the scanned offset
 // boff[t] in (a, then b) order.
 //
-// One event a (level index t) walking its successors until the input state changes: the form for
-// states whose events carry no position masks (parents past 63 edges; the test compares edge ids).
-template <bool kEmit>
-__device__ void bpairs_walk(const DevPtrs& P, const LevelArgs& A, uint32_t t) {
-    const uint32_t a = A.ev_base + t;
-    const uint32_t end = A.ev_base + A.n_events;
-    uint32_t cnt = 0;
-    if (P.ev_kept[a]) {
-        const uint32_t in = P.ev_in[a];
-        const uint32_t na = P.rules[P.ev_rule[a]].n_lhs, ca0 = P.ev_coff[a];
-        const unsigned long long ma = P.ev_bmask[a];
-        uint32_t ca[kMaxPatternEdges];   // edge ids, for parents past the mask's 63 positions
-        bool have_ca = false;
-        uint32_t out = kEmit ? A.boff[t] : 0u;
-        for (uint32_t c = a + 1; c < end && P.ev_in[c] == in; ++c) {
-            const unsigned long long mc = P.ev_bmask[c];
-            bool share = false;
-            if (ma && mc) {
-                // a consumed parent position in common (never with a dropped event's mask)
-                share = (ma & mc) != 0ull;
-            } else if (P.ev_kept[c]) {
-                if (!have_ca) {
-                    for (uint32_t k = 0; k < na; ++k) ca[k] = P.ev_cons[ca0 + k];
-                    have_ca = true;
-                }
-                const uint32_t nc = P.rules[P.ev_rule[c]].n_lhs, cc0 = P.ev_coff[c];
-                for (uint32_t k = 0; k < nc && !share; ++k) {
-                    const uint32_t x = P.ev_cons[cc0 + k];
-                    for (uint32_t m = 0; m < na; ++m) share |= (ca[m] == x);
-                }
-            }
-            if (!share) continue;
-            if (kEmit) reinterpret_cast<uint2*>(A.bpairs)[out++] = make_uint2(a, c);
-            ++cnt;
-        }
-    }
-    if (!kEmit) A.bcount[t] = cnt;
-}
-
-// Thread per event of the level whose parent carries no position masks (more than 63 edges; then
-// none of its events has one): the per-event walk. The other events are k_bpairs'.
+// Parents of more than 63 edges: thread per event, walking the state's later events until the input
+// state changes. A pair's masks are tested first; only pairs whose masks meet are compared by edge
+// ids (5.1 ms with the ids of every pair, 3.3 with the masks, over 129 evolutions of 65-256-edge
+// states). One warp per state instead, as below, took 37 ms there: few states with thousands of events.
 template <bool kEmit>
 __global__ void k_bpairs_walk(DevPtrs P, LevelArgs A) {
-    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < A.n_events; t += gridDim.x * blockDim.x)
-        if (P.ev_bmask[A.ev_base + t] == 0ull) bpairs_walk<kEmit>(P, A, t);
+    const uint32_t end = A.ev_base + A.n_events;
+    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < A.n_events; t += gridDim.x * blockDim.x) {
+        const uint32_t a = A.ev_base + t, in = P.ev_in[a];
+        if (P.st_ne[in] <= 63) continue;   // k_bpairs'
+        uint32_t cnt = 0;
+        const unsigned long long ma = P.ev_kept[a] ? P.ev_bmask[a] : 0ull;
+        uint32_t out = kEmit ? A.boff[t] : 0u;
+        if (ma)
+            for (uint32_t c = a + 1; c < end && P.ev_in[c] == in; ++c) {
+                if ((ma & P.ev_bmask[c]) == 0ull || !share_edge(P, a, c)) continue;
+                if (kEmit) reinterpret_cast<uint2*>(A.bpairs)[out++] = make_uint2(a, c);
+                ++cnt;
+            }
+        if (!kEmit) A.bcount[t] = cnt;
+    }
 }
 
-// Warp per input state (frontier position f, events [item_ev[f R], item_ev[(f+1) R]) of the
-// level) whose events carry position masks (a parent of at most 63 edges; a dropped event carries
-// kMaskDropped): lane i holds the mask of event i of a 32-event tile and takes the masks of the
+// Warp per input state (frontier position f, events [item_ev[f R], item_ev[(f+1) R]) of the level)
+// of at most 63 edges: lane i holds the mask of event i of a 32-event tile and takes the masks of the
 // later events from the other lanes by shuffles, so every pair test is one AND of registers.
 template <bool kEmit>
 __global__ void k_bpairs(DevPtrs P, LevelArgs A) {
@@ -2933,7 +3224,7 @@ __global__ void k_bpairs(DevPtrs P, LevelArgs A) {
         if (g1 <= g0) continue;
         const uint32_t k = g1 - g0;
         const uint32_t e0 = A.ev_base + g0;
-        if (P.ev_bmask[e0] == 0ull) continue;   // no masks: k_bpairs_walk's
+        if (P.st_ne[A.frontier[f]] > 63) continue;   // k_bpairs_walk's
         for (uint32_t t0 = 0; t0 < k; t0 += 32) {
             const uint32_t i = t0 + lane;
             const bool mine = i < k;

@@ -66,8 +66,8 @@ struct DevPtrs {
     // transitive reduction: per event, bit d set = an event at level d is a proper causal
     // ancestor (levels < 64; an event's ancestors lie on its input state's history chain)
     unsigned long long* ev_anc;
-    // per event: the parent positions it consumed as a bit mask for the branchial test, or 0 when
-    // the parent has more than 63 edges (compare edge ids); bit 63 alone: the event is not kept
+    // per event: the parent positions it consumed as a bit mask for the branchial test (branch_mask);
+    // bit 63 alone: the event is not kept
     unsigned long long* ev_bmask;
     // event canonicalisation: per event its signature; per evolution the distinct signatures
     unsigned long long* ev_sig;
@@ -86,6 +86,9 @@ struct LevelArgs {
     uint32_t n_frontier;
     uint32_t rules_stride;      // R: item (f, r) = f * R + r
     uint32_t* counts;           // [F*R] matches per item
+    uint32_t* chunks;           // [F*R*kChunks] matches from every 32 first edges of a large state, or
+                                // null
+    uint32_t parts;             // warps that count a large state together
     uint32_t* item_ev;          // [F*R+1] exclusive scans
     uint32_t* item_cons;
     uint32_t* item_prod;
@@ -98,7 +101,7 @@ struct LevelArgs {
     const uint32_t* frng;
     uint32_t n_frng;
     // warp-per-child kernel: exclusive scan over the n_sw work indices of their parents' slice
-    // counts (soff[n_sw] = total); a slice is a run of slice_size(children) consecutive children
+    // counts (soff[n_sw] = total); a slice is a run of wslice consecutive children
     const uint32_t* soff;
     uint32_t n_sw;
     uint8_t* fmode;             // [F] bit 0: within the lane path's limits; bit 1: forwarding;
@@ -107,7 +110,7 @@ struct LevelArgs {
     uint32_t ev_keys;           // event signature keys (0 = no event canonicalisation)
     uint32_t lane_vmax;         // largest child (vertices) of this level the lane path takes
     uint32_t path;              // the level's small-state kernel as its fmode bit: 1 lane, 4 segment
-    uint32_t slice;             // segment kernel: most children of a work unit
+    uint32_t slice, wslice;     // segment and warp-per-child kernels: most children of a work unit
     uint32_t* work;             // work-queue counters
     // select / assign
     uint32_t* flag_new;         // [n_events]
@@ -129,12 +132,14 @@ struct LevelArgs {
 
 // Per-warp shared-memory carve-up, sized on the host from the level's largest state.
 struct Layout {
-    uint32_t NE, NOCC, CNE, CNOCC, V, W, NBR;
+    uint32_t NE, NOCC, CNE, CNOCC, V, W;
+    uint32_t LH;        // left-hand edges of the longest rule (match list stride)
+    uint32_t BUF;       // warp WL: neighbour words in shared memory
     uint32_t NV;        // distinct vertices a staged state may have (V = NV + fresh variables)
-    uint32_t o_cur, o_nxt, o_csum, o_ccnt, o_nbr;                  // u64
-    uint32_t o_peid, o_occ, o_ooff, o_nbo, o_deg, o_nn, o_comp;     // u32
+    uint32_t o_cur, o_nxt, o_buf;                                   // u64
+    uint32_t o_peid, o_ooff, o_deg, o_nn, o_comp, o_glob, o_first;  // u32
     uint32_t o_cand, o_taken, o_misc;                               // u32
-    uint32_t o_pevo, o_vloc, o_cvo, o_bind, o_match, o_mdepth;      // u16
+    uint32_t o_pevo, o_vloc, o_cvo, o_bind, o_match, o_mdepth, o_mpos, o_occ;   // u16
     uint32_t o_pear, o_car;                                         // u8
     uint32_t o_rule;                                                // DevRule
     // lane-per-child path: parent occurrence and neighbour lists by vertex, per-vertex degree /
@@ -156,7 +161,6 @@ struct Layout {
     // SEGN neighbour entries, produced edges per batch slot
     uint32_t o_ppk, o_seg, SEGB, SEGE, SEGN, RHS;
     uint32_t VT, o_vtab, o_vtid;   // vertex hash table for large states (VT slots, 0 = unused)
-    uint32_t o_srt;                // warp WL: sort buffer of the distinct-colour count
     // join indices of a staged state past kJoinIndexMin edges (XI = 1; count and warp layouts):
     // vertex -> state positions of the edges holding it (CSR), and the edges bucketed by
     // signature (at most kSigBuckets buckets); o_xready: bit 0 vertex index, bit 1 signature index

@@ -107,3 +107,36 @@ def test_record_options_and_serving_steps(engines):
             eng.set_option(api.OPT_RECORD_BRANCHIAL, True)
         for i, (a, b) in enumerate(zip(*out)):
             same_arrays(a, b, (causal, branchial, i))
+
+
+@pytest.mark.parametrize("n", [31, 33, 319, 321, 640, 641, 700])
+def test_hub_vertex_hashes(engines, n):
+    """One vertex in n edges: its neighbour words pass the registers' 32 and the buffer's 640 (an
+    arity-3 hub twice as early), its occurrences the buffer of a mixed-arity state's first colours."""
+    from oracle import pyoracle
+    star = [[1, i + 2] for i in range(n)]
+    roots = [star, [e + [e[1] % 7 + 2] for e in star], star + [[1], [1], [2, 3, 1]],
+             [[1]] * n + star[: n // 2], [[1, 1]] * (n // 2) + [[1, 2]]]
+    res = engines[0].evolve([([[0, 1]], [[0, 1]])], roots, 0, quotient=False)
+    assert [int(h) for h in res.state_hash] == [pyoracle.wl_hash(r) for r in roots]
+
+
+@pytest.mark.parametrize("arity,n_lhs", [(2, 2), (3, 2), (2, 3), (2, 5)])
+def test_large_state_joins(engines, arity, n_lhs):
+    """States of 65-130 edges: index walks (rules of up to four left-hand edges) and the warp join
+    against the oracle, with and without the join index."""
+    from oracle import pyoracle
+    rng = W.SplitMix64(41 + arity + n_lhs)
+    lhs = [[k] + [k + 1] * (arity - 1) if k % 2 else [k + 1] + [k] * (arity - 1) for k in range(n_lhs)]
+    rule = (lhs, [[n_lhs, 0] + [n_lhs + 1] * (arity - 2), [n_lhs + 1] * arity])
+    for edges in (65, 97, 130):
+        root = W.random_hypergraph(rng, edges, arity) + [[5] * arity, [6] * arity]
+        ref = pyoracle.evolve([rule], [root], 2, quotient=True, max_states=60)
+        want = pyoracle.normalize(ref["state_hash"], ref["events"], ref["causal"], ref["branchial"])
+        for index in (1, 0):
+            engines[0].set_option(api.OPT_JOIN_INDEX, index)
+            res = engines[0].evolve([rule], [root], 2, quotient=True, max_states=60)
+            got = pyoracle.normalize(res.state_hash, res.events, res.causal, res.branchial)
+            for k in want:
+                assert np.array_equal(got[k], want[k]), (edges, index, k)
+        engines[0].set_option(api.OPT_JOIN_INDEX, 1)
