@@ -174,6 +174,8 @@ __host__ __device__ inline uint32_t align_up(uint32_t x, uint32_t a) { return (x
 
 // A streamed result's level is split into parts of at least this many frontier states.
 constexpr uint32_t kStreamPartStates = 16384;
+// ... the last level of a run also into parts of about this many events.
+constexpr uint32_t kStreamPartEvents = 1u << 17;
 // Smallest level (children) of small binary states that the lane kernel takes from the segment one.
 constexpr uint32_t kLaneLevel = 1u << 20;
 // Results streamed only when the last one was at least this large (a small result's copy is
@@ -257,7 +259,10 @@ __host__ __device__ Layout make_layout(uint32_t NE, uint32_t NOCC, const RuleMax
     if (!lane) next_use();   // (the lane layouts go on using the scratch)
     L.o_cand = take(4 * kMaxPatternEdges * L.W, 4);
     L.VM = std::min<uint32_t>(L.NV, lane ? kLaneVMax : 64);
-    L.o_vm = take(8 * L.VM, 8);
+    // (the lane layouts: in load_parent's scratch, 8 NOCC bytes: the lane kernel's local arrays live in
+    // what the blocks' shared memory leaves of L1. 4 KB a block for these masks and a vertex table
+    // sized by occurrences cost C2's largest levels 7.2 against 6.2 ms)
+    L.o_vm = lane ? u0 : take(8 * L.VM, 8);
     if (index && !lane && NE > kJoinIndexMin) {
         L.XI = 1;
         L.o_xoff = take(4 * (NOCC + 1), 4);
@@ -876,6 +881,7 @@ struct Engine::Impl {
     uint64_t n_states = 0, n_edges = 0, n_events = 0, n_cons = 0, n_bpairs = 0;
     uint64_t next_vertex = 0, arena_words = 0, tab_slots = 0;
     uint32_t frontier_size = 0;
+    uint32_t levels_done = 0;   // levels since the run began
     uint32_t ne_bound = 1, nocc_bound = 1;
     bool uniform = true;      // each evolution's roots and right-hand sides share one arity, 2 or 3
     uint64_t run_ne = 1, run_no = 1;   // the run's largest state record so far (edges, occurrences)
@@ -1006,6 +1012,7 @@ struct Engine::Impl {
         n_roots_admitted = 0;
         next_vertex = arena_words = tab_slots = 0;
         frontier_size = 0;
+        levels_done = 0;
         ne_bound = nocc_bound = 1;
         run_ne = run_no = 1;
         uniform = true;
@@ -1389,6 +1396,7 @@ struct Engine::Impl {
         G.tab0 = tab0;
         G.tab1 = tab_slots;
         G.arena_words = arena_words;
+        G.one_root = nr == nnew ? 1u : 0u;   // (every evolution has at least one)
         G.fresh = fresh_run ? 1u : 0u;
         fresh_run = false;
         const uint64_t most = std::max<uint64_t>({tab_slots - tab0, words.size(), rule_words, batch_edges, 256});
@@ -1409,8 +1417,10 @@ struct Engine::Impl {
         k_roots<<<sh.grid, sh.block, sh.smem, st>>>(ptrs(), root_ids.p, nr, work.p, L);
         check_launch();
         hist.have_ok = false;   // the roots move the class and state counters
-        k_root_counts<<<grid_for(nr, 256), 256, 0, st>>>(ptrs(), root_ids.p, nr);
-        check_launch();
+        if (nr != nnew) {   // (one root each: k_admit set the counters)
+            k_root_counts<<<grid_for(nr, 256), 256, 0, st>>>(ptrs(), root_ids.p, nr);
+            check_launch();
+        }
         toc(times.roots);
         frontier_size += static_cast<uint32_t>(h_front.size());
         return ids;
@@ -1511,7 +1521,7 @@ struct Engine::Impl {
     // whose four synchronisations no longer count. Measured per call with the one-launch
     // admission, before and after: C1 of two steps (3 KB) 567 -> 358 us, C1 (4.7 MB) 1,224 -> 1,011 us.
     // Empty (no flat arrays) when the bound is larger.
-    static constexpr uint64_t kFinSmallBytes = 16ull << 20;
+    static constexpr uint64_t kFinSmallBytes = 16ull << 20, kFinDirectBytes = 32ull << 10;
     EvolutionResult finalize_small(const RunOptions& opt) {
         EvolutionResult r;
         const bool se = opt.keep_state_edges, si = se && opt.keep_state_edge_ids, sg = opt.event_keys != 0;
@@ -1549,12 +1559,19 @@ struct Engine::Impl {
         const unsigned long long* hs = sync_host(ResultArrays::kArrays + 4);
         F.head = d_sync;
         F.host = h;
-        k_fin_small_sums<<<G, 256, 0, st>>>(ptrs(), F);
-        check_launch();
+        // a few hundred records: the emission's one block sums for itself and writes straight to the
+        // host block (one launch; C1 of two steps 211 -> 209 us a call)
+        if (total <= kFinDirectBytes) F.stage = h;
+        if (G > 1) {
+            k_fin_small_sums<<<G, 256, 0, st>>>(ptrs(), F);
+            check_launch();
+        }
         k_fin_small_emit<<<G, 256, 0, st>>>(ptrs(), F);
         check_launch();
-        k_fin_small_copy<<<copy_grid(total), 256, 0, st>>>(F);
-        check_launch();
+        if (total > kFinDirectBytes) {
+            k_fin_small_copy<<<copy_grid(total), 256, 0, st>>>(F);
+            check_launch();
+        }
         sync_st();
         uint64_t at = 0;
         for (int i = 0; i < ResultArrays::kArrays; ++i) {
@@ -2109,6 +2126,7 @@ struct Engine::Impl {
             hist.have[1] = o[6] | (uint64_t(o[7]) << 32);
             hist.stopped = o[8];
             done += n;
+            levels_done += n;
             if (n) grown = false;
             if (sr.on && n) {
                 const uint32_t q[7] = {uint32_t(e_old), uint32_t(n_events), uint32_t(s_old), uint32_t(n_states),
@@ -2175,7 +2193,12 @@ struct Engine::Impl {
         // the level's frontier ranges: [0, P), in up to four parts when the result streams (each
         // part's share of the result is copied out while the next computes), then [P, F)
         std::vector<std::pair<uint32_t, uint32_t>> parts;
-        const uint32_t K = sr.on ? std::min<uint32_t>(4, std::max<uint32_t>(1, P / kStreamPartStates)) : 1;
+        uint32_t K = sr.on ? std::min<uint32_t>(4, std::max<uint32_t>(1, P / kStreamPartStates)) : 1;
+        // the run's last level has no later one to hide its copy behind: parts by the events to expect
+        // (C2 to 7 levels, whose last level is 989,694 events of 24,700 states: one part 7.0 ms a call,
+        // four 6.1 ms)
+        if (sr.on && nevo == 1 && levels_done + 1 == h_evos[0].steps && hist.valid)
+            K = std::max(K, std::min<uint32_t>(4, static_cast<uint32_t>(hist.ev_per_state * P / kStreamPartEvents)));
         for (uint32_t j = 0; j < K; ++j)
             parts.emplace_back(uint32_t(uint64_t(P) * j / K), uint32_t(uint64_t(P) * (j + 1) / K));
         if (P < F) parts.emplace_back(P, F);
@@ -2218,6 +2241,7 @@ struct Engine::Impl {
                 evo_done[e] = 1;
                 finished.push_back(static_cast<uint32_t>(e));
             }
+        ++levels_done;
         std::swap(frontier, next_frontier);
         frontier_size = sub_nf;
         ne_bound = static_cast<uint32_t>(sub_ne);
@@ -2388,7 +2412,7 @@ struct Engine::Impl {
         if (n_ev) {
             const uint32_t mne = std::max<uint32_t>(fmax_ne, 1), mno = std::max<uint32_t>(fmax_nocc, 1);
             const Layout Ll = make_layout(std::min<uint32_t>(mne, kLaneEMax), mno, rm, LayoutKind::Lane, fwd,
-                                          fmax_cnt);
+                                          fmax_cnt, false, fmax_nv);
             const Layout Lw = make_layout(mne, mno, rm, LayoutKind::Warp, fwd, kLaneJoinCap,
                                           opt.join_index != 0, fmax_nv);
             // matches by lane walks; the warp join where it is asked for (rules of more than four

@@ -1766,6 +1766,7 @@ struct AdmitArgs {
     uint64_t edges0, edges1;  // initial edges (no producer)
     uint64_t tab0, tab1;      // dedup table slots
     uint64_t arena_words;     // the arena's top after this batch
+    uint32_t one_root;        // every evolution has one root: one class, one state
     uint32_t fresh;           // first admission of a run: clear the error flags and counters
 };
 
@@ -1797,9 +1798,9 @@ __global__ void k_admit(DevPtrs P, AdmitArgs G) {
     }
     for (uint64_t i = t; i < G.n_evos; i += stride) {
         const uint64_t e = G.evo0 + i;
-        P.evo_classes[e] = 0;
+        P.evo_classes[e] = G.one_root;
         P.evo_causal[e] = 0;
-        P.evo_states[e] = 0;
+        P.evo_states[e] = G.one_root;
         P.evo_sigs[e] = 0;
         P.evo_cut[e] = kNone;
         P.evo_stopped[e] = 0;
@@ -3490,8 +3491,8 @@ __device__ __forceinline__ uint32_t causal_of(const DevPtrs& P, uint32_t e) {
     return c;
 }
 
-__global__ void __launch_bounds__(256) k_fin_small_sums(DevPtrs P, FinSmall F) {
-    __shared__ uint32_t sh[3];
+// This block's totals (causal triples, state edges, occurrences) into sh[0..2].
+__device__ void fin_small_totals(const DevPtrs& P, const FinSmall& F, uint32_t* sh) {
     if (threadIdx.x < 3) sh[threadIdx.x] = 0;
     __syncthreads();
     const uint32_t G = gridDim.x, b = blockIdx.x;
@@ -3513,7 +3514,12 @@ __global__ void __launch_bounds__(256) k_fin_small_sums(DevPtrs P, FinSmall F) {
         atomicAdd(&sh[2], no);
     }
     __syncthreads();
-    if (threadIdx.x < 3) F.sums[threadIdx.x * G + b] = sh[threadIdx.x];
+}
+
+__global__ void __launch_bounds__(256) k_fin_small_sums(DevPtrs P, FinSmall F) {
+    __shared__ uint32_t sh[3];
+    fin_small_totals(P, F, sh);
+    if (threadIdx.x < 3) F.sums[threadIdx.x * gridDim.x + blockIdx.x] = sh[threadIdx.x];
 }
 
 __global__ void __launch_bounds__(256) k_fin_small_emit(DevPtrs P, FinSmall F) {
@@ -3521,7 +3527,10 @@ __global__ void __launch_bounds__(256) k_fin_small_emit(DevPtrs P, FinSmall F) {
     __shared__ uint64_t off[kArr], count[kArr];
     __shared__ uint32_t ebase[256], vbase[256];
     const uint32_t G = gridDim.x, b = blockIdx.x, tid = threadIdx.x, lane = lane_id();
-    if (tid < 96) {   // warp a: array a's prefix before this block and its total
+    if (G == 1) {   // one block: its own totals
+        fin_small_totals(P, F, all);
+        if (tid < 3) pre[tid] = 0;
+    } else if (tid < 96) {   // warp a: array a's prefix before this block and its total
         const uint32_t a = tid >> 5;
         uint32_t p = 0, t = 0;
         for (uint32_t i = lane; i < G; i += 32) {
