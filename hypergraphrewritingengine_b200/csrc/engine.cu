@@ -256,7 +256,7 @@ __host__ __device__ Layout make_layout(uint32_t NE, uint32_t NOCC, const RuleMax
         L.o_vtab = take(4 * L.VT, 4);
         L.o_vtid = take(2 * L.VT, 2);
     }
-    if (!lane) next_use();   // (the lane layouts go on using the scratch)
+    next_use();
     L.o_cand = take(4 * kMaxPatternEdges * L.W, 4);
     L.VM = std::min<uint32_t>(L.NV, lane ? kLaneVMax : 64);
     // (the lane layouts: in load_parent's scratch, 8 NOCC bytes: the lane kernel's local arrays live in
@@ -288,10 +288,8 @@ __host__ __device__ Layout make_layout(uint32_t NE, uint32_t NOCC, const RuleMax
         L.BUF = std::max<uint32_t>(std::min<uint32_t>(L.CNOCC * std::max<uint32_t>(rm.arity - 1, 1), +kWlBuf), n2 + 1);
         L.o_buf = take(8 * L.BUF, 8);
     }
-    if (!lane) {
-        next_use();
-        off = u1;
-    }
+    next_use();
+    off = u1;
     if (kind == LayoutKind::Seg) {
         L.o_ppk = take(4 * NE, 4);
         L.RHS = rm.rhs;

@@ -226,13 +226,15 @@ HGX_HD uint64_t lane_wl_core(const uint8_t* pear, const uint16_t* pevo, const ui
     info.nocc = nocc;
     info.nbr = nbr;
     if (nv == 0) return 0;
-    // produced occurrences by vertex: bit p of pm[v] <=> RHS position p holds v (ascending p is
-    // RHS edge order, then position order)
-    uint64_t pm[VM];
+    // produced occurrences by vertex: bit p of pm[v] <=> RHS position p < 32 holds v (ascending p is
+    // RHS edge order, then position order); later positions are looked for where they are needed
+    // (32 bits, not 64: the array is local memory, and the kernel lives off L1)
+    uint32_t pm[VM];
         #pragma unroll 1
     for (uint32_t v = 0; v < V; ++v) pm[v] = 0;
+    const uint32_t rt32 = R.rhs_total < 32 ? R.rhs_total : 32u;
         #pragma unroll 1
-    for (uint32_t p = 0; p < R.rhs_total; ++p) pm[prodv[p]] |= 1ull << p;
+    for (uint32_t p = 0; p < rt32; ++p) pm[prodv[p]] |= 1u << p;
 
     uint64_t cura[VM], curb[VM], buf[NM];
     uint64_t* cur = cura;   // this round's colours
@@ -264,10 +266,16 @@ HGX_HD uint64_t lane_wl_core(const uint8_t* pear, const uint16_t* pevo, const ui
             buf[n++] = (static_cast<uint64_t>(pear[e]) << 8) | (x & 15u);
         }
                 #pragma unroll 1
-        for (uint64_t m = pm[v]; m && n < cap; m &= m - 1) {
+        for (uint32_t m = pm[v]; m && n < cap; m &= m - 1) {
             const uint32_t p = lane_ctz64(m), k = R.rhs_pos_edge[p];
             buf[n++] = (static_cast<uint64_t>(R.rhs_ar[k]) << 8) | (p - R.rhs_off[k]);
         }
+                #pragma unroll 1
+        for (uint32_t p = 32; p < R.rhs_total && n < cap; ++p)
+            if (prodv[p] == v) {
+                const uint32_t k = R.rhs_pos_edge[p];
+                buf[n++] = (static_cast<uint64_t>(R.rhs_ar[k]) << 8) | (p - R.rhs_off[k]);
+            }
         lane_isort64(buf, n);
         uint64_t h = fnv(kFnvOffset, static_cast<uint64_t>(dn[v] & 0xFFFFu));
                 #pragma unroll 1
@@ -293,9 +301,17 @@ HGX_HD uint64_t lane_wl_core(const uint8_t* pear, const uint16_t* pevo, const ui
                 buf[n++] = fnv(cur[(x >> 4) & 63u], x & 15u);
             }
                         #pragma unroll 1
-            for (uint64_t m = pm[v]; m; m &= m - 1) {
+            for (uint32_t m = pm[v]; m; m &= m - 1) {
                 const uint32_t p = lane_ctz64(m), kk = R.rhs_pos_edge[p];
                 const uint32_t a = R.rhs_ar[kk], o = R.rhs_off[kk], q = p - o;
+                                #pragma unroll 1
+                for (uint32_t t = 0; t < a; ++t)
+                    if (t != q) buf[n++] = fnv(cur[prodv[o + t]], t);
+            }
+                        #pragma unroll 1
+            for (uint32_t p = 32; p < R.rhs_total; ++p) {
+                if (prodv[p] != v) continue;
+                const uint32_t kk = R.rhs_pos_edge[p], a = R.rhs_ar[kk], o = R.rhs_off[kk], q = p - o;
                                 #pragma unroll 1
                 for (uint32_t t = 0; t < a; ++t)
                     if (t != q) buf[n++] = fnv(cur[prodv[o + t]], t);

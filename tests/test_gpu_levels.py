@@ -140,3 +140,19 @@ def test_large_state_joins(engines, arity, n_lhs):
             for k in want:
                 assert np.array_equal(got[k], want[k]), (edges, index, k)
         engines[0].set_option(api.OPT_JOIN_INDEX, 1)
+
+
+def test_long_right_hand_sides(engines):
+    """Right-hand sides of more than 32 positions (15 binary edges and a ternary one) in the lane and
+    warp kernels, against the oracle."""
+    from oracle import pyoracle
+    rhs = [[k % 3, (k + 1) % 4] for k in range(15)] + [[0, 1, 2]]
+    rules = [([[0, 1], [1, 2]], rhs), ([[0, 1, 2]], [[0, 1], [1, 2]])]
+    roots = [[[1, 2], [2, 3], [3, 1]]]
+    ref = pyoracle.evolve(rules, roots, 2, quotient=True)
+    want = pyoracle.normalize(ref["state_hash"], ref["events"], ref["causal"], ref["branchial"])
+    for eng in engines:
+        res = eng.evolve(rules, roots, 2, quotient=True)
+        got = pyoracle.normalize(res.state_hash, res.events, res.causal, res.branchial)
+        for k in want:
+            assert np.array_equal(got[k], want[k]), k
