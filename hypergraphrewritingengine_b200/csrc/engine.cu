@@ -225,7 +225,11 @@ __host__ __device__ Layout make_layout(uint32_t NE, uint32_t NOCC, const RuleMax
     L.o_match = take(2 * kMaxPatternEdges, 2);
     L.o_mdepth = take(2 * kMaxPatternEdges, 2);
     L.LH = rm.lhs;
-    if (wl) L.o_mpos = take(2 * rm.lhs * kListMax, 2);
+    if (wl) {
+        L.o_mpos = take(2 * rm.lhs * kListMax, 2);
+        L.o_ppk = take(4 * std::min<uint32_t>(NE, +kSegEMax), 4);
+        L.o_sprod = take(4 * kMaxPatternEdges, 4);
+    }
     L.o_pear = take(NE, 1);
     if (wl) L.o_car = take(L.CNE, 1);
     L.o_rule = take(sizeof(DevRule), 4);
@@ -287,6 +291,13 @@ __host__ __device__ Layout make_layout(uint32_t NE, uint32_t NOCC, const RuleMax
         while (n2 < 2 * L.V) n2 <<= 1;
         L.BUF = std::max<uint32_t>(std::min<uint32_t>(L.CNOCC * std::max<uint32_t>(rm.arity - 1, 1), +kWlBuf), n2 + 1);
         L.o_buf = take(8 * L.BUF, 8);
+    }
+    if (wl) {   // or those of a small state of one arity hashed by seg_wl
+        next_use();
+        const uint32_t a = rm.arity < 3 ? 2 : 3;
+        L.SEGE = std::min<uint32_t>(L.CNE, +kSegEMax);
+        L.SEGN = L.SEGE * a * (a - 1);
+        L.o_seg = take(seg_scratch_bytes(32, L.SEGE, L.SEGN), 8);
     }
     next_use();
     off = u1;
@@ -1238,7 +1249,8 @@ struct Engine::Impl {
         uint64_t max_label = 0;
         // dedup table slots per evolution: enough for its small levels without a rehash (32,768 for a
         // single one, cleared in 2 us), a million slots over a batch, at least 256 each
-        uint64_t table_slots = 32768;
+        // (256 each under a device-memory ceiling, which they could otherwise reach before the run does)
+        uint64_t table_slots = budget.limit ? 256 : 32768;
         while (table_slots > 256 && table_slots * specs.size() > (1u << 20)) table_slots >>= 1;
         for (size_t i = 0; i < specs.size(); ++i) {
             const EvolutionSpec& spec = *specs[i];
@@ -1995,7 +2007,7 @@ struct Engine::Impl {
             // not worth a look: too many items, or more events than the limit to expect (each state of
             // E edges has about E matches or more: a batch's large roots would be counted in vain), or
             // by the last level's events per state
-            if (uint64_t(frontier_size) * rm.stride > kFusedItems || uint64_t(frontier_size) * ne_bound > 2 * kFusedEvents ||
+            if (uint64_t(frontier_size) * rm.stride > kFusedItems || uint64_t(frontier_size) * ne_bound > 32768 ||
                 (nevo == 1 && hist.valid && hist.ev_per_state * frontier_size > kFusedEvents))
                 break;
             const uint32_t levels = std::min<uint32_t>({most - done, kFusedLevels,
@@ -2291,7 +2303,7 @@ struct Engine::Impl {
                                       opt.join_index != 0);
         fmode.ensure(F, 0, st);
         A.fmode = fmode.p;
-        if (ne_bound > uint32_t(kLaneEMax)) {
+        if (ne_bound > uint32_t(kLaneEMax) && !budget.limit) {
             chunks.ensure(items * kChunks, 0, st);
             A.chunks = chunks.p;
         }

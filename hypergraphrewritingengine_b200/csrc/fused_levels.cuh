@@ -83,9 +83,15 @@ struct FusedArgs {
 constexpr uint32_t kReportWords = 32;
 
 // Grid barrier of a cooperative launch; the last block to arrive runs `serial` before the others are
-// released. Returns false when the wait ran out (an error flag is set; every block then leaves).
+// released. Returns false when a wait ran out: the waiter then closes the barrier for everyone --
+// release and closing are one compare-and-swap on the same word, so either all blocks pass it or all
+// leave, the late ones included. Up to the end of the expansion nothing of a level counts yet (its
+// table inserts repeat themselves with the same ids), so a level whose joins or hashes take one block
+// longer than the wait is simply run again by the ordinary pipeline; later it is an error (`hard`).
+constexpr uint32_t kBarrierClosed = 0xFFFFFFFFu;
+
 template <class F>
-__device__ bool fused_barrier(FusedState* fs, uint32_t& phase, uint32_t* err, F&& serial) {
+__device__ bool fused_barrier(FusedState* fs, uint32_t& phase, uint32_t* err, bool hard, F&& serial) {
     __shared__ uint32_t sh_last, sh_ok;
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -94,7 +100,6 @@ __device__ bool fused_barrier(FusedState* fs, uint32_t& phase, uint32_t* err, F&
         sh_ok = 1;
     }
     __syncthreads();
-    ++phase;
     if (sh_last) {
         if (threadIdx.x == 0) __threadfence();
         __syncthreads();
@@ -102,24 +107,24 @@ __device__ bool fused_barrier(FusedState* fs, uint32_t& phase, uint32_t* err, F&
         __syncthreads();
         if (threadIdx.x == 0) {
             __threadfence();
-            atomicExch(&fs->gen, phase);
+            sh_ok = atomicCAS(&fs->gen, phase, phase + 1) == phase ? 1u : 0u;
         }
-        __syncthreads();
-        return true;
-    }
-    if (threadIdx.x == 0) {
-        uint32_t g = 0, it = 0;
-        for (; it < (1u << 22); ++it) {   // about two seconds
+    } else if (threadIdx.x == 0) {
+        uint32_t g = phase;
+        for (uint32_t it = 0; g == phase && it < (1u << 22); ++it)   // about two seconds
             asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(g) : "l"(&fs->gen) : "memory");
-            if (g >= phase) break;
+        if (g == phase) {
+            g = atomicCAS(&fs->gen, phase, kBarrierClosed);
+            if (g == phase) {
+                g = kBarrierClosed;
+                if (hard) atomicOr(err, kErrBarrier);
+            }
         }
-        if (g < phase) {
-            sh_ok = 0;
-            atomicOr(err, kErrBarrier);
-        }
+        sh_ok = g == phase + 1 ? 1u : 0u;
         __threadfence();
     }
     __syncthreads();
+    ++phase;
     return sh_ok != 0;
 }
 
@@ -163,7 +168,9 @@ __device__ uint32_t fused_pairs(const DevPtrs& P, uint32_t a, uint32_t end, uint
 __global__ void __launch_bounds__(kFusedThreads, 1) k_levels(DevPtrs P, FusedArgs G) {
     extern __shared__ __align__(16) char smem[];
     __shared__ Layout L;
+    __shared__ SegTables tables;
     __shared__ uint32_t sh[33], pre[3], all[3];
+    seg_tables_fill(tables);
     const uint32_t tid = threadIdx.x, lane = lane_id(), w = tid >> 5;
     const uint32_t nb = gridDim.x, b = blockIdx.x;
     FusedState* fs = G.fs;
@@ -233,7 +240,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_levels(DevPtrs P, FusedArg
         }
         // ---- barrier 1: scans, per-evolution checks, the decision
         uint32_t* ranges = range_out + uint64_t(lv) * G.nevo * kRangeWords;
-        alive = fused_barrier(fs, phase, P.err, [&] {
+        alive = fused_barrier(fs, phase, P.err, false, [&] {
             fused_scan(G.item_ev, NI, sh);
             fused_scan(G.item_cons, NI, sh);
             fused_scan(G.item_prod, NI, sh);
@@ -328,6 +335,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_levels(DevPtrs P, FusedArg
             uint32_t staged = kNone;
             Parent pa{0, 0, 0};
             bool pconn = false;
+            uint32_t ar = 0;   // the staged parent's one arity (2 or 3), or 0
             for (uint32_t t = lo_t, x = x0; x < x1; ++t) {
                 const uint32_t t0 = G.item_ev[t], rn = G.cnt[t];
                 if (x >= t0 + rn) continue;   // an item without events
@@ -338,20 +346,29 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_levels(DevPtrs P, FusedArg
                     staged = f;
                     pa = load_parent(P, L, sm, sid);
                     pconn = parent_connected(L, sm, pa);
+                    // one arity of 2 or 3, and the packed edges seg_wl reads
+                    const uint8_t* pear = smp<uint8_t>(sm, L.o_pear);
+                    const uint32_t a0 = pa.ne ? pear[0] : 0u;
+                    bool one = (a0 == 2 || a0 == 3) && pa.ne <= kSegEMax && pa.nvp <= 32;
+                    for (uint32_t k = lane; k < pa.ne; k += 32) one = one && pear[k] == a0;
+                    ar = __all_sync(0xFFFFFFFFu, one) ? a0 : 0u;
+                    if (ar)
+                        for (uint32_t k = lane; k < pa.ne; k += 32) {
+                            const uint16_t* v = smp<uint16_t>(sm, L.o_vloc) + smp<uint16_t>(sm, L.o_pevo)[k];
+                            smp<uint32_t>(sm, L.o_ppk)[k] = v[0] | (uint32_t(v[1]) << 8) | (ar == 3 ? uint32_t(v[2]) << 16 : 0u);
+                        }
+                    __syncwarp();
                     if (lane == 0 && t0 == x) b_hbm += 4ull * (pa.ne + (pa.ne + 3) / 4 + pa.nocc) + 20;
                 }
                 load_rule(sm, L, &P.rules[ev.rule_begin + r]);
                 const uint32_t cons0 = n_cons + G.item_cons[t], prod0 = n_edges + G.item_prod[t],
                                fresh0 = next_vertex + G.item_fresh[t];
                 const uint32_t lo = x - t0, hi = min(rn, x1 - t0);
-                auto child = [&](uint32_t idx, uint32_t nm) {
-                    uint8_t rpos[kMaxPatternEdges];
-                    for (uint32_t k = 0; k < Rr.n_lhs; ++k) rpos[k] = static_cast<uint8_t>(match[k]);
-                    const uint32_t nec = build_child(L, sm, Rr, pa, nm);
-                    WlInfo info;
-                    const uint64_t h = warp_wl(L, sm, nec, pa.nvp + Rr.n_fresh, info,
-                                               pconn && (Rr.flags & kRuleRhsJoinsLhs));
+                // one child's event record and table insert
+                auto record = [&](uint32_t idx, uint64_t h, const WlInfo& info, const uint16_t* pos, uint32_t nec) {
                     if (lane == 0) {
+                        uint8_t rpos[kMaxPatternEdges];
+                        for (uint32_t k = 0; k < Rr.n_lhs; ++k) rpos[k] = static_cast<uint8_t>(pos[k]);
                         const uint32_t e = ev_base + t0 + idx, coff = cons0 + idx * Rr.n_lhs,
                                        pid = prod0 + idx * Rr.n_rhs;
                         P.ev_in[e] = sid;
@@ -361,7 +378,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_levels(DevPtrs P, FusedArg
                         P.ev_fresh[e] = fresh0 + idx * Rr.n_fresh;
                         P.ev_hash[e] = h;
                         P.ev_nv[e] = info.nv;
-                        for (uint32_t k = 0; k < Rr.n_lhs; ++k) P.ev_cons[coff + k] = peid[match[k]];
+                        for (uint32_t k = 0; k < Rr.n_lhs; ++k) P.ev_cons[coff + k] = peid[pos[k]];
                         P.ev_bmask[e] = branch_mask(Rr.n_lhs, pa.ne, rpos);
                         for (uint32_t k = 0; k < Rr.n_rhs; ++k) P.edge_creator[pid + k] = e;
                         table_insert(P, ev, h, e);
@@ -378,21 +395,67 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_levels(DevPtrs P, FusedArg
                     }
                     __syncwarp();
                 };
+                const bool joined = pconn && (Rr.flags & kRuleRhsJoinsLhs);
                 // the run's matches listed, then one child after another
                 const Fwd none{};
                 const uint16_t* mpos = smp<uint16_t>(sm, L.o_mpos);
-                uint32_t* taken = smp<uint32_t>(sm, L.o_taken);
-                if (list_matches(P, L, sm, Rr, pa, none, lo, hi, rn)) {
+                if (!list_matches(P, L, sm, Rr, pa, none, lo, hi, rn)) {
+                } else if (ar && (Rr.rhs_uni == ar || !Rr.n_rhs) && pa.nvp + Rr.n_fresh <= 32 &&
+                           pa.ne + Rr.n_rhs <= kSegEMax + Rr.n_lhs) {
+                    // small states of one arity: hashed from the staged edges, no child is built
+                    const uint32_t* ppk = smp<uint32_t>(sm, L.o_ppk);
+                    uint32_t* sprod = smp<uint32_t>(sm, L.o_sprod);
+                    const uint16_t* pevo = smp<uint16_t>(sm, L.o_pevo);
+                    const uint16_t* vloc = smp<uint16_t>(sm, L.o_vloc);
+                    const uint32_t keep = pa.ne - Rr.n_lhs;
+                    for (uint32_t i = lo; i < hi; ++i) {
+                        const uint16_t* pos = mpos + (i - lo) * L.LH;
+                        unsigned long long rm = 0;
+                        for (uint32_t k = 0; k < Rr.n_lhs; ++k) rm |= 1ull << pos[k];
+                        if (lane < Rr.n_rhs) {   // lane k packs produced edge k
+                            uint32_t pk = 0;
+                            for (uint32_t q = 0; q < ar; ++q) {
+                                const uint32_t var = Rr.rhs_vars[Rr.rhs_off[lane] + q];
+                                uint32_t x = pa.nvp + Rr.fresh_rank[var];
+                                if (!((Rr.new_mask >> var) & 1u)) {   // its first place on the left
+                                    uint32_t k = 0, p = 0;
+                                    while (Rr.lhs_vars[Rr.lhs_off[k] + p] != var)
+                                        if (++p == Rr.lhs_ar[k]) { ++k; p = 0; }
+                                    x = vloc[pevo[pos[k]] + p];
+                                }
+                                pk |= x << (8 * q);
+                            }
+                            sprod[lane] = pk;
+                        }
+                        __syncwarp();
+                        WlInfo info;
+                        const uint64_t h = seg_wl<32>(keep + Rr.n_rhs, 32, ar, joined, sm + L.o_seg, L.SEGE, L.SEGN,
+                                                      tables, [&](uint32_t j) -> uint32_t {
+                            if (j >= keep) return sprod[j - keep];
+                            uint32_t p = j;   // the j-th kept edge: past every removed position at or before it
+                            for (unsigned long long m = rm; m; m &= m - 1)
+                                p += p >= static_cast<uint32_t>(__ffsll(static_cast<long long>(m)) - 1) ? 1u : 0u;
+                            return ppk[p];
+                        }, info);
+                        record(i, h, info, pos, keep + Rr.n_rhs);
+                    }
+                } else {
+                    uint32_t* taken = smp<uint32_t>(sm, L.o_taken);
                     for (uint32_t k = lane; k < L.W; k += 32) taken[k] = 0;
                     __syncwarp();
                     for (uint32_t i = lo; i < hi; ++i)
-                        fwd_emit(L, sm, Rr, mpos + (i - lo) * L.LH, [&](uint32_t nm) { child(i, nm); });
+                        fwd_emit(L, sm, Rr, mpos + (i - lo) * L.LH, [&](uint32_t nm) {
+                            const uint32_t nec = build_child(L, sm, Rr, pa, nm);
+                            WlInfo info;
+                            const uint64_t h = warp_wl(L, sm, nec, pa.nvp + Rr.n_fresh, info, joined);
+                            record(i, h, info, match, nec);
+                        });
                 }
                 if (lane == 0 && lo == 0) b_stage += 4ull * pa.ne + 4ull * pa.nocc;
                 x = t0 + hi;
             }
         }
-        alive = fused_barrier(fs, phase, P.err, [] {});
+        alive = fused_barrier(fs, phase, P.err, false, [] {});
         if (!alive) break;
         // ---- select: this thread's event from here to the end of the level
         const uint32_t ec = (n_ev + nb - 1) / nb;
@@ -434,7 +497,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_levels(DevPtrs P, FusedArg
         const uint32_t f_at = block_excl_scan(front ? 1u : 0u, sh, tot[1]);
         const uint32_t b_at = block_excl_scan(bc, sh, tot[2]);
         if (tid < 3) G.sums[tid * nb + b] = tot[tid];
-        alive = fused_barrier(fs, phase, P.err, [] {});
+        alive = fused_barrier(fs, phase, P.err, true, [] {});
         if (!alive) break;
         // ---- assign
         if (w < 3) {
@@ -515,7 +578,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_levels(DevPtrs P, FusedArg
         ne_b = mne + G.rm.grow_e;
         no_b = mno + G.rm.grow_o;
         cur ^= 1;
-        alive = fused_barrier(fs, phase, P.err, [] {});
+        alive = fused_barrier(fs, phase, P.err, true, [] {});
         if (!alive) break;
         // ---- output states (the next count reads none of it)
         bool swin = false;
@@ -541,11 +604,11 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_levels(DevPtrs P, FusedArg
     __syncthreads();
     if (tid == 0) {
         __threadfence();
-        // blocks that left at a timed-out barrier still arrive here once
+        // (blocks that left at a closed barrier arrive here once, like the others)
         if (atomicAdd(&fs->abort, 1u) + 1 == nb) {
             __threadfence();
             volatile uint32_t* o = G.out;
-            o[0] = __ldcg(&fs->stop);
+            o[0] = __ldcg(&fs->gen) == kBarrierClosed ? uint32_t(kStopLevel) : __ldcg(&fs->stop);
             o[1] = lv;
             o[2] = cur;
             o[3] = __ldcg(P.err);

@@ -159,7 +159,7 @@ struct Layout {
     uint32_t SB;                                                    // bytes per batch slot
     // segment path: packed parent edges, per-segment scratch for states of at most SEGE edges and
     // SEGN neighbour entries, produced edges per batch slot
-    uint32_t o_ppk, o_seg, SEGB, SEGE, SEGN, RHS;
+    uint32_t o_ppk, o_sprod, o_seg, SEGB, SEGE, SEGN, RHS;
     uint32_t VT, o_vtab, o_vtid;   // vertex hash table for large states (VT slots, 0 = unused)
     // join indices of a staged state past kJoinIndexMin edges (XI = 1; count and warp layouts):
     // vertex -> state positions of the edges holding it (CSR), and the edges bucketed by

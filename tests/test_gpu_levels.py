@@ -156,3 +156,22 @@ def test_long_right_hand_sides(engines):
         got = pyoracle.normalize(res.state_hash, res.events, res.causal, res.branchial)
         for k in want:
             assert np.array_equal(got[k], want[k]), k
+
+
+def test_noalloc_states_at_the_segment_limits():
+    """hgx_hash_states_noalloc on both of its kernels: 31-33 vertices, 63-65 edges, one arity of 1 to 4
+    and mixed ones, components, a hub, and labels at the ends of their range."""
+    import test_zz_no_alloc as Z
+    from hypergraphrewritingengine_b200 import load_library
+    from oracle import pyoracle
+    states = []
+    for arity in (1, 2, 3, 4):
+        for nv in (1, 2, 16, 17, 31, 32, 33):
+            for ne in (1, 2, 31, 32, 33, 63, 64, 65):
+                states.append([[(k * (q + 1) + q) % nv for q in range(arity)] for k in range(ne)])
+    states += [[[1, 2], [2, 3, 4]], [[1, 2], [3, 4], [5, 6]], [[0, 2], [3, 0]], [[0xFFFFFFFE, 5], [5, 0xFFFFFFFE]],
+               [[7, k] for k in range(8, 39)], [[7, k, 7] for k in range(8, 39)], [[3, 3], [3, 3], [4, 3]]]
+    h, cls = Z._noalloc(load_library(), states)
+    want = [pyoracle.wl_hash(s) for s in states]
+    assert [int(x) for x in h] == want
+    assert [int(c) for c in cls] == [want.index(x) for x in want]
