@@ -368,8 +368,6 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_levels(DevPtrs P, FusedArg
                 // one child's event record and table insert
                 auto record = [&](uint32_t idx, uint64_t h, const WlInfo& info, const uint16_t* pos, uint32_t nec) {
                     if (lane == 0) {
-                        uint8_t rpos[kMaxPatternEdges];
-                        for (uint32_t k = 0; k < Rr.n_lhs; ++k) rpos[k] = static_cast<uint8_t>(pos[k]);
                         const uint32_t e = ev_base + t0 + idx, coff = cons0 + idx * Rr.n_lhs,
                                        pid = prod0 + idx * Rr.n_rhs;
                         P.ev_in[e] = sid;
@@ -380,7 +378,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_levels(DevPtrs P, FusedArg
                         P.ev_hash[e] = h;
                         P.ev_nv[e] = info.nv;
                         for (uint32_t k = 0; k < Rr.n_lhs; ++k) P.ev_cons[coff + k] = peid[pos[k]];
-                        P.ev_bmask[e] = branch_mask(Rr.n_lhs, pa.ne, rpos);
+                        P.ev_bmask[e] = branch_mask(Rr.n_lhs, pa.ne, pos);
                         for (uint32_t k = 0; k < Rr.n_rhs; ++k) P.edge_creator[pid + k] = e;
                         table_insert(P, ev, h, e);
                         const uint64_t k = Rr.n_lhs, rr = Rr.n_rhs;

@@ -1942,7 +1942,8 @@ __global__ void k_item_sizes(DevPtrs P, LevelArgs A) {
 // kMaskDropped, which has no bit in common with any other mask.
 constexpr unsigned long long kMaskDropped = 1ull << 63;
 
-__device__ __forceinline__ unsigned long long branch_mask(uint32_t n, uint32_t pne, const uint8_t* pos) {
+template <class Pos>   // bytes in the batches of small states, 16 bits for the others
+__device__ __forceinline__ unsigned long long branch_mask(uint32_t n, uint32_t pne, const Pos* pos) {
     unsigned long long m = 0;
     for (uint32_t k = 0; k < n; ++k) m |= 1ull << (pne > 63 ? pos[k] % 63u : pos[k]);
     return m;
@@ -2048,8 +2049,9 @@ __global__ void __launch_bounds__(256, 3) k_expand(DevPtrs P, LevelArgs A, Layou
             const uint32_t rule_g = ev.rule_begin + r;
             if (!kLane && (fm & 2u)) build_join_index(L, sm, pa);   // for the seeded joins
             const Fwd fwd = fwd_prepare(P, A, L, sm, R, ev, pa, sid, (fm & 2u) != 0);
-            // per-child work shared by both paths: the event record and the table insert
-            auto finish = [&](uint32_t idx, uint64_t h, const WlInfo& info, const uint8_t* rpos) {
+            // per-child work shared by both paths: the event record and the table insert (rpos: the
+            // consumed positions, bytes on the lane path, 16 bits on the other)
+            auto finish = [&](uint32_t idx, uint64_t h, const WlInfo& info, const auto* rpos) {
                 const uint32_t e = ev0 + idx;
                 const uint32_t coff = cons0 + idx * R.n_lhs;
                 const uint32_t pid = prod0 + idx * R.n_rhs;
@@ -2163,15 +2165,13 @@ __global__ void __launch_bounds__(256, 3) k_expand(DevPtrs P, LevelArgs A, Layou
                 uint32_t* taken = smp<uint32_t>(sm, L.o_taken);
                 for (uint32_t k = lane; k < L.W; k += 32) taken[k] = 0;
                 __syncwarp();
-                uint8_t rpos[kMaxPatternEdges];
                 for (uint32_t idx = lo; idx < hi; ++idx)
                     fwd_emit(L, sm, R, mpos + (idx - lo) * L.LH, [&](uint32_t nm) {
-                        for (uint32_t k = 0; k < R.n_lhs; ++k) rpos[k] = static_cast<uint8_t>(match[k]);
                         const uint32_t nec = build_child(L, sm, R, pa, nm);
                         WlInfo info;
                         const uint64_t h = warp_wl(L, sm, nec, pa.nvp + R.n_fresh, info,
                                                    pconn && (R.flags & kRuleRhsJoinsLhs));
-                        if (lane == 0) finish(idx, h, info, rpos);
+                        if (lane == 0) finish(idx, h, info, match);
                         __syncwarp();
                     });
             }

@@ -1,0 +1,57 @@
+"""Evolutions of states past 256 edges (positions of more than a byte) against the oracle."""
+import numpy as np
+import pytest
+
+from hypergraphrewritingengine_b200 import Engine, api
+from oracle import pyoracle
+from parity import assert_same, norm_gpu, norm_oracle
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def eng():
+    e = Engine(0)
+    yield e
+    e.close()
+
+
+def _edges(res, s):
+    """The edges of state s as the result stores them."""
+    e0, e1 = res.state_edge_off[s: s + 2]
+    ends = res.state_vert_off[s] + np.cumsum(res.state_arity[e0:e1].astype(np.int64))
+    return [v.tolist() for v in np.split(res.state_verts[res.state_vert_off[s]: ends[-1]],
+                                         (ends - res.state_vert_off[s])[:-1])]
+
+
+def _chain(n):
+    return [[i, i + 1] for i in range(1, n)] + [[n, 1]]
+
+
+# loops, then edges out of the first loops' vertices: the only matches of the rule hold the
+# positions p and p + 256
+LOOPS = [[i, i] for i in range(1, 257)] + [[i, 1000 + i] for i in range(1, 25)]
+CASES = {
+    "chain-255": (([[0, 1], [1, 2]], [[0, 1], [1, 2], [2, 0]]), _chain(255), True, 20),
+    "chain-256": (([[0, 1], [1, 2]], [[0, 1], [1, 2], [2, 0]]), _chain(256), True, 20),
+    "chain-257": (([[0, 1], [1, 2]], [[0, 1], [1, 2], [2, 0]]), _chain(257), True, 20),
+    "chain-300": (([[0, 1], [1, 2]], [[2, 0]]), _chain(300), False, 700),
+    "chain-520": (([[0, 1], [1, 2]], [[0, 1], [1, 2], [2, 0]]), _chain(520), True, 5),
+    "p-and-p+256": (([[0, 0], [0, 1]], [[0, 1], [1, 2]]), LOOPS, False, 0),
+    "five-lhs-260": (([[0, 1], [1, 2], [2, 3], [3, 4], [4, 5]], [[0, 5], [5, 6]]), _chain(260), False, 300),
+}
+
+
+@pytest.mark.parametrize("forwarding", [0, 1])
+@pytest.mark.parametrize("name", sorted(CASES))
+def test_positions_past_a_byte(eng, name, forwarding):
+    rule, root, quotient, cap = CASES[name]
+    eng.set_option(api.OPT_FORWARDING, forwarding)
+    res = eng.evolve([rule], [root], 2, quotient=quotient, max_states=cap)
+    eng.set_option(api.OPT_FORWARDING, 0)
+    ref = pyoracle.evolve([rule], [root], 2, quotient=quotient, max_states=cap)
+    assert_same(norm_gpu(res), norm_oracle(ref), name)
+    # a stored state is the one its hash was taken of
+    for s in sorted({0, 1, 7, len(res.state_hash) // 2, len(res.state_hash) - 1}):
+        if s < len(res.state_hash):
+            assert pyoracle.wl_hash(_edges(res, s)) == int(res.state_hash[s]), (name, s)
