@@ -239,6 +239,10 @@ hgx_status hgx_engine_set_option(hgx_engine* e, hgx_option opt, uint64_t value) 
             if (value > 2) return fail(HGX_ERR_INVALID, "stream result: 0 off, 1 results of 64 MB or more, 2 always");
             e->opt.stream_result = static_cast<uint32_t>(value);
             return HGX_OK;
+        case HGX_OPT_HASTY_BARRIER:
+            if (value > 64) return fail(HGX_ERR_INVALID, "hasty barrier: 0 none, or 1 to 64");
+            e->opt.hasty_barrier = static_cast<uint32_t>(value);
+            return HGX_OK;
         case HGX_OPT_LANE_JOIN:
             if (value > 2) return fail(HGX_ERR_INVALID, "lane join must be 0 (default), 1 or 2");
             e->opt.lane_join = static_cast<uint32_t>(value);

@@ -2076,6 +2076,7 @@ struct Engine::Impl {
             G.tr = opt.transitive_reduction;
             G.branchial = opt.branchial;
             G.index = opt.join_index;
+            G.hasty = opt.hasty_barrier - 1;   // (0: none)
             G.rm = rm;
             // shared memory for a full block of warps a few levels on, within the launch's limit (a
             // larger state has fewer warps a block, down to one)

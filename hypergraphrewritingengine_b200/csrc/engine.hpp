@@ -113,6 +113,9 @@ struct RunOptions {
     // at the end); 2 = the same whatever the size; 0 = the whole result is copied at the end.
     // Identical results.
     uint32_t stream_result = 1;
+    // Tests: the n-th grid barrier (from 1) of a launch of small levels is given up after one look, as
+    // one whose wait runs out (four barriers a level); 0: none.
+    uint32_t hasty_barrier = 0;
 };
 
 // Per-stage device time of the last run (CUDA events on the engine stream), milliseconds.

@@ -75,6 +75,7 @@ struct FusedArgs {
     uint32_t n_states, n_events, n_edges, n_cons, next_vertex;      // totals so far
     uint32_t F, stride, nevo, levels, ne_bound, no_bound, smem;
     uint32_t ev_keys, tr, branchial, index;
+    uint32_t hasty;             // barrier given up after one look, kNone: none
     RuleMax rm;
 };
 
@@ -84,15 +85,18 @@ struct FusedArgs {
 constexpr uint32_t kReportWords = 32;
 
 // Grid barrier of a cooperative launch; the last block to arrive runs `serial` before the others are
-// released. Returns false when a wait ran out: the waiter then closes the barrier for everyone --
-// release and closing are one compare-and-swap on the same word, so either all blocks pass it or all
-// leave, the late ones included. Up to the end of the expansion nothing of a level counts yet (its
+// released. gen counts the barriers passed. Returns false when a wait ran out: the waiter then closes
+// the barrier for everyone -- release and closing are one compare-and-swap on the same word, so either
+// all blocks pass it or all leave, the late ones included. The closed word keeps the count below it: a
+// block still waiting at an earlier barrier sees that it was released, finishes its part of that level
+// and leaves where the others do. Up to the end of the expansion nothing of a level counts yet (its
 // table inserts repeat themselves with the same ids), so a level whose joins or hashes take one block
 // longer than the wait is simply run again by the ordinary pipeline; later it is an error (`hard`).
-constexpr uint32_t kBarrierClosed = 0xFFFFFFFFu;
+// `hasty`: the barrier (of the launch, from 0) that is given up after one look (for tests).
+constexpr uint32_t kBarrierClosed = 1u << 31;
 
 template <class F>
-__device__ bool fused_barrier(FusedState* fs, uint32_t& phase, uint32_t* err, bool hard, F&& serial) {
+__device__ bool fused_barrier(FusedState* fs, uint32_t& phase, uint32_t* err, bool hard, uint32_t hasty, F&& serial) {
     __shared__ uint32_t sh_last, sh_ok;
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -112,16 +116,14 @@ __device__ bool fused_barrier(FusedState* fs, uint32_t& phase, uint32_t* err, bo
         }
     } else if (threadIdx.x == 0) {
         uint32_t g = phase;
-        for (uint32_t it = 0; g == phase && it < (1u << 22); ++it)   // about two seconds
+        const uint32_t looks = phase == hasty ? 1u : 1u << 22;   // about two seconds
+        for (uint32_t it = 0; g == phase && it < looks; ++it)
             asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(g) : "l"(&fs->gen) : "memory");
         if (g == phase) {
-            g = atomicCAS(&fs->gen, phase, kBarrierClosed);
-            if (g == phase) {
-                g = kBarrierClosed;
-                if (hard) atomicOr(err, kErrBarrier);
-            }
+            g = atomicCAS(&fs->gen, phase, phase | kBarrierClosed);
+            if (g == phase && hard) atomicOr(err, kErrBarrier);
         }
-        sh_ok = g == phase + 1 ? 1u : 0u;
+        sh_ok = (g & ~kBarrierClosed) > phase ? 1u : 0u;
         __threadfence();
     }
     __syncthreads();
@@ -241,7 +243,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_levels(DevPtrs P, FusedArg
         }
         // ---- barrier 1: scans, per-evolution checks, the decision
         uint32_t* ranges = range_out + uint64_t(lv) * G.nevo * kRangeWords;
-        alive = fused_barrier(fs, phase, P.err, false, [&] {
+        alive = fused_barrier(fs, phase, P.err, false, G.hasty, [&] {
             fused_scan(G.item_ev, NI, sh);
             fused_scan(G.item_cons, NI, sh);
             fused_scan(G.item_prod, NI, sh);
@@ -454,7 +456,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_levels(DevPtrs P, FusedArg
                 x = t0 + hi;
             }
         }
-        alive = fused_barrier(fs, phase, P.err, false, [] {});
+        alive = fused_barrier(fs, phase, P.err, false, G.hasty, [] {});
         if (!alive) break;
         // ---- select: this thread's event from here to the end of the level
         const uint32_t ec = (n_ev + nb - 1) / nb;
@@ -496,7 +498,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_levels(DevPtrs P, FusedArg
         const uint32_t f_at = block_excl_scan(front ? 1u : 0u, sh, tot[1]);
         const uint32_t b_at = block_excl_scan(bc, sh, tot[2]);
         if (tid < 3) G.sums[tid * nb + b] = tot[tid];
-        alive = fused_barrier(fs, phase, P.err, true, [] {});
+        alive = fused_barrier(fs, phase, P.err, true, G.hasty, [] {});
         if (!alive) break;
         // ---- assign
         if (w < 3) {
@@ -577,7 +579,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_levels(DevPtrs P, FusedArg
         ne_b = mne + G.rm.grow_e;
         no_b = mno + G.rm.grow_o;
         cur ^= 1;
-        alive = fused_barrier(fs, phase, P.err, true, [] {});
+        alive = fused_barrier(fs, phase, P.err, true, G.hasty, [] {});
         if (!alive) break;
         // ---- output states (the next count reads none of it)
         bool swin = false;
@@ -607,7 +609,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_levels(DevPtrs P, FusedArg
         if (atomicAdd(&fs->abort, 1u) + 1 == nb) {
             __threadfence();
             volatile uint32_t* o = G.out;
-            o[0] = __ldcg(&fs->gen) == kBarrierClosed ? uint32_t(kStopLevel) : __ldcg(&fs->stop);
+            o[0] = (__ldcg(&fs->gen) & kBarrierClosed) ? uint32_t(kStopLevel) : __ldcg(&fs->stop);
             o[1] = lv;
             o[2] = cur;
             o[3] = __ldcg(P.err);

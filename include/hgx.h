@@ -125,7 +125,12 @@ typedef enum hgx_option {
        overlap the evolution; page-locked blocks are sized from that previous result, and a result
        that outgrows them is copied whole at the end); 2 = the same for results of any size; 0 =
        the whole result is copied after the last level. Identical results. The reference reads its result back after the last step (gpu/src/evolve.cu:489-496). */
-    HGX_OPT_STREAM_RESULT = 16
+    HGX_OPT_STREAM_RESULT = 16,
+    /* For tests: the n-th grid barrier (1 to 64; four to a level) of a launch of small levels is
+       given up after one look at its word, as a barrier whose wait (about two seconds) runs out.
+       At the first two of a level the level is run again by the ordinary pipeline with identical
+       results; at the others the call fails with HGX_ERR_INTERNAL. 0 (default): none. */
+    HGX_OPT_HASTY_BARRIER = 17
 } hgx_option;
 
 /* One evolution of a batch or a served request. */

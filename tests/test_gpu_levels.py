@@ -175,3 +175,35 @@ def test_noalloc_states_at_the_segment_limits():
     want = [pyoracle.wl_hash(s) for s in states]
     assert [int(x) for x in h] == want
     assert [int(c) for c in cls] == [want.index(x) for x in want]
+
+
+@pytest.mark.parametrize("barrier", [1, 2, 5, 6, 9, 13, 14])
+def test_a_barrier_that_closes_leaves_the_level_to_the_ordinary_pipeline(engines, barrier):
+    """A level's first two barriers run out: the launch ends there for every block -- also for one that
+    is still on its way out of the barrier before (5, 9, 13: the first of a later level) -- and the
+    level is run again over the tables it has partly filled."""
+    rules, roots, steps, quotient, cap = SINGLE["ternary-5"]
+    want = engines[1].evolve(rules, roots, steps, quotient=quotient, max_states=cap)
+    engines[0].evolve(rules, roots, steps, quotient=quotient, max_states=cap)
+    usual = engines[0].stage_times()[1]
+    engines[0].set_option(api.OPT_HASTY_BARRIER, barrier)
+    try:
+        for _ in range(20):
+            same_arrays(engines[0].evolve(rules, roots, steps, quotient=quotient, max_states=cap), want, barrier)
+            assert engines[0].stage_times()[1] > usual   # (launches: the repeated level's)
+    finally:
+        engines[0].set_option(api.OPT_HASTY_BARRIER, 0)
+
+
+@pytest.mark.parametrize("barrier", [3, 4, 8])
+def test_a_barrier_that_closes_after_the_expansion_fails_the_call(engines, barrier):
+    rules, roots, steps, quotient, cap = SINGLE["ternary-5"]
+    want = engines[1].evolve(rules, roots, steps, quotient=quotient, max_states=cap)
+    engines[0].set_option(api.OPT_HASTY_BARRIER, barrier)
+    try:
+        with pytest.raises(api.HgxError) as err:
+            engines[0].evolve(rules, roots, steps, quotient=quotient, max_states=cap)
+        assert err.value.status == api.HGX_ERR_INTERNAL
+    finally:
+        engines[0].set_option(api.OPT_HASTY_BARRIER, 0)
+    same_arrays(engines[0].evolve(rules, roots, steps, quotient=quotient, max_states=cap), want, barrier)
