@@ -18,7 +18,7 @@ CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libhgx.so")
 SOURCES = ["engine.cu", "capi.cpp"]
 DEPS = ["engine.cu", "capi.cpp", "engine.hpp", "step_kernels.cu", "step_kernels.cuh", "common.cuh",
-        "lane_wl.cuh", "fused_levels.cuh", "seg_wl.cuh", "seg_expand.cuh",
+        "lane_wl.cuh", "fused_levels.cuh", "fused_rule.cuh", "seg_wl.cuh", "seg_expand.cuh",
         os.path.join("..", "..", "include", "hgx.h")]
 
 

@@ -12,6 +12,7 @@
 
 #include "../../include/hgx.h"
 
+#include "fused_rule.cuh"
 #include "step_kernels.cu"
 
 namespace hgx {
@@ -2010,6 +2011,8 @@ struct Engine::Impl {
             if (uint64_t(frontier_size) * rm.stride > kFusedItems || uint64_t(frontier_size) * ne_bound > 32768 ||
                 (nevo == 1 && hist.valid && hist.ev_per_state * frontier_size > kFusedEvents))
                 break;
+            // (the launch counts in 32 bits from here on)
+            if (std::max({n_events, n_states, n_cons, n_edges, next_vertex}) >= kIdLimit) break;
             const uint32_t levels = std::min<uint32_t>({most - done, kFusedLevels,
                                                         std::max<uint32_t>(1, static_cast<uint32_t>(4096 / nevo))});
             const size_t words = kReportWords + kFusedLevels * kLevelWords + size_t(levels) * nevo * kRangeWords;
@@ -2051,13 +2054,13 @@ struct Engine::Impl {
                                               state_of_arrival.cap, ev_bmask.cap});
             if (opt.transitive_reduction) re = std::min<uint64_t>(re, ev_anc.cap);
             if (opt.event_keys) re = std::min<uint64_t>(re, ev_sig.cap);
-            G.room_events = re;
-            G.room_states = std::min<uint64_t>({st_off.cap, st_hash.cap, st_ne.cap, st_nocc.cap, st_evo.cap,
+            G.room.events = re;
+            G.room.states = std::min<uint64_t>({st_off.cap, st_hash.cap, st_ne.cap, st_nocc.cap, st_evo.cap,
                                                 st_depth.cap, st_event.cap, st_ev0.cap, st_evn.cap, st_nv.cap});
-            G.room_cons = std::min<uint64_t>(ev_cons.cap, ev_cprod.cap);
-            G.room_edges = edge_creator.cap;
-            G.room_pairs = bpairs.cap / 2;
-            G.room_arena = arena.cap;
+            G.room.cons = std::min<uint64_t>(ev_cons.cap, ev_cprod.cap);
+            G.room.edges = edge_creator.cap;
+            G.room.pairs = bpairs.cap / 2;
+            G.room.arena = arena.cap;
             G.room_front = static_cast<uint32_t>(std::min<uint64_t>({frontier.cap, next_frontier.cap, new_state_event.cap, 0xFFFFFFFFull}));
             G.arena_words = arena_words;
             G.n_pairs = n_bpairs;

@@ -33,23 +33,12 @@
 #pragma once
 
 constexpr uint32_t kFusedThreads = 512, kFusedWarps = kFusedThreads / 32;
-constexpr uint32_t kFusedEvents = 16384;    // most events of a level (a thread per event, 148 blocks)
 constexpr uint32_t kFusedItems = 8192;      // most (state, rule) items of a level: one block scans them
 constexpr uint32_t kFusedLevels = 16;       // most levels of a launch (records in mapped memory)
-constexpr uint32_t kFusedEdges = 255;       // largest state record a level may produce
 constexpr uint32_t kFusedSlice = kListMax;  // most events a warp builds in one run
 static_assert(kFusedEvents <= kNumSMs * kFusedThreads, "one event per thread");
 constexpr uint32_t kRangeWords = 10;        // per level and evolution: see k_levels
 constexpr uint32_t kLevelWords = 8;         // per level: F, events, states, frontier, pairs, max ne / nocc
-
-// Why a level was left to the ordinary pipeline.
-enum FusedStop : uint32_t {
-    kStopDone = 0,          // no frontier left, or the level count asked for
-    kStopRoom = 1,          // an array has no room: grow and come back
-    kStopLevel = 2,         // too many events or items, or a cap that can bind
-    kStopTable = 3,         // a dedup table would pass half full
-    kStopLayout = 4,        // a state's shared-memory region does not fit
-};
 
 // Grid-wide words of the launch (zero between launches: the last block to leave clears them).
 struct FusedState {
@@ -68,10 +57,10 @@ struct FusedArgs {
     uint32_t* bpairs;
     uint32_t* evo_last;         // per evolution: one past its last event of the level
     uint32_t* out;              // mapped: header, level records, ranges
-    uint64_t room_events, room_states, room_cons, room_edges, room_pairs, room_arena;   // array sizes
+    FusedSizes room;            // array sizes
     uint64_t arena_words;       // bound of the arena's bump pointer
     uint64_t n_pairs;
-    uint32_t room_front, room_items;
+    uint32_t room_front;
     uint32_t n_states, n_events, n_edges, n_cons, next_vertex;      // totals so far
     uint32_t F, stride, nevo, levels, ne_bound, no_bound, smem;
     uint32_t ev_keys, tr, branchial, index;
@@ -250,18 +239,13 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_levels(DevPtrs P, FusedArg
             fused_scan(G.item_fresh, NI, sh);
             const uint32_t n_ev = G.item_ev[NI];
             if (tid == 0) {
-                uint32_t stop = kStopDone;
                 const uint64_t mne = uint64_t(fs->max_ne[par]) + G.rm.grow_e, mno = uint64_t(fs->max_no[par]) + G.rm.grow_o;
                 const uint64_t rec = mne + (mne + 3) / 4 + mno;
-                if (W == 0) stop = kStopLayout;
-                else if (n_ev > kFusedEvents || mne > kFusedEdges) stop = kStopLevel;
-                else if (uint64_t(n_events) + n_ev > G.room_events || uint64_t(n_states) + n_ev > G.room_states ||
-                         uint64_t(n_cons) + G.item_cons[NI] > G.room_cons ||
-                         uint64_t(n_edges) + G.item_prod[NI] > G.room_edges ||
-                         (G.branchial && n_pairs + fs->pairs[par] > G.room_pairs) ||
-                         arena_words + n_ev * rec > G.room_arena || n_ev > G.room_front)
-                    stop = kStopRoom;
-                else if (uint64_t(next_vertex) + G.item_fresh[NI] >= 0xFFFFFFF0ull) stop = kStopLevel;
+                const FusedSizes have{n_events, n_states, n_cons, n_edges, next_vertex, n_pairs, arena_words};
+                const FusedSizes level{n_ev, n_ev, G.item_cons[NI], G.item_prod[NI], G.item_fresh[NI], fs->pairs[par],
+                                       n_ev * rec};
+                uint32_t stop = W == 0 ? uint32_t(kStopLayout)
+                                       : fused_decide(have, level, G.room, G.room_front, mne, G.branchial != 0);
                 if (!stop) {
                     const Layout Lw = make_layout(max(fs->max_ne[par], 1u), max(fs->max_no[par], 1u), G.rm,
                                                   LayoutKind::Warp, false, kLaneJoinCap, G.index != 0,

@@ -2,7 +2,8 @@
 
 The expand kernel's lane-per-child WL hash (csrc/lane_wl.cuh) is a __host__ __device__
 function; tests/native/lane_wl_test.cpp compiles it for the host and checks it against the
-oracle's WL hash on random parents and matches (AddressSanitizer on).
+oracle's WL hash on random parents and matches (AddressSanitizer on). The rule by which a level runs
+inside the launch of small levels (csrc/fused_rule.cuh) is checked at its limits.
 """
 import os
 import shutil
@@ -26,6 +27,15 @@ def test_lane_wl_matches_oracle(tmp_path):
     assert int(out.stdout.split("(")[1].split()[0]) > 1000, out.stdout
     # children hashed through the uniform-arity initial colours (counts by position)
     assert int(out.stdout.split(", ")[1].split()[0]) > 1000, out.stdout
+
+
+@pytest.mark.skipif(shutil.which("g++") is None, reason="needs g++")
+def test_fused_level_rule(tmp_path):
+    exe = tmp_path / "fused_rule_test"
+    subprocess.check_call(["g++", "-std=c++17", "-O1", "-fsanitize=address", "-I", ROOT,
+                           os.path.join(ROOT, "tests", "native", "fused_rule_test.cpp"), "-o", str(exe)])
+    out = subprocess.run([str(exe)], capture_output=True, text=True, timeout=60)
+    assert out.returncode == 0, out.stdout + out.stderr
 
 
 def _build_compat(tmp_path):
