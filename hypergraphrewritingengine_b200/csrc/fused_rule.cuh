@@ -14,13 +14,17 @@ namespace hgx {
 
 constexpr uint32_t kFusedEvents = 16384;    // most events of a level (a thread per event, 148 blocks)
 constexpr uint32_t kFusedEdges = 255;       // largest state record a level may produce
+// Most branchial pairs to make room for ahead of a level. The launch has no count of them before it
+// writes them, only the bound c (c - 1) / 2 of every state with c matches: 8 MB at this limit, 1 GB for
+// one state of 16,384 matches, of which the ordinary level, which counts first, needs a few percent.
+constexpr uint64_t kFusedPairs = 1u << 20;
 constexpr uint64_t kIdLimit = 0xFFFFFFF0ull;   // 32-bit ids end here
 
 // Why a level was left to the ordinary pipeline.
 enum FusedStop : uint32_t {
     kStopDone = 0,          // no frontier left, or the level count asked for
     kStopRoom = 1,          // an array has no room: grow and come back
-    kStopLevel = 2,         // too many events or items, a cap that can bind, ids that run out
+    kStopLevel = 2,         // too many events, items or pairs, a cap that can bind, ids that run out
     kStopTable = 3,         // a dedup table would pass half full
     kStopLayout = 4,        // a state's shared-memory region does not fit
 };
@@ -36,6 +40,7 @@ struct FusedSizes {
 HGX_RULE uint32_t fused_decide(const FusedSizes& have, const FusedSizes& level, const FusedSizes& room,
                                uint64_t room_front, uint64_t largest_record, bool branchial) {
     if (level.events > kFusedEvents || largest_record > kFusedEdges) return kStopLevel;
+    if (branchial && level.pairs > kFusedPairs) return kStopLevel;
     if (have.events + level.events >= kIdLimit || have.states + level.events >= kIdLimit ||
         have.cons + level.cons >= kIdLimit || have.edges + level.edges >= kIdLimit ||
         have.vertices + level.vertices >= kIdLimit || (branchial && have.pairs + level.pairs >= kIdLimit))

@@ -55,6 +55,13 @@ int main() {
     expect("too many events", decide(none, wide, room), kStopLevel);
     expect("largest record", decide(none, level, room, 1 << 20, kFusedEdges), kStopDone);
     expect("record too large", decide(none, level, room, 1 << 20, kFusedEdges + 1), kStopLevel);
+    wide = level;
+    wide.pairs = kFusedPairs;
+    expect("most pairs", decide(none, wide, room), kStopDone);
+    wide.pairs = kFusedPairs + 1;
+    expect("too many pairs", decide(none, wide, room), kStopLevel);
+    expect("too many pairs before room", decide(none, wide, {big, big, big, big, big, 10, big}), kStopLevel);
+    expect("pairs that are not kept", decide(none, wide, room, 1 << 20, 10, false), kStopDone);
     std::printf("%d wrong\n", bad);
     return bad != 0;
 }

@@ -207,3 +207,14 @@ def test_a_barrier_that_closes_after_the_expansion_fails_the_call(engines, barri
     finally:
         engines[0].set_option(api.OPT_HASTY_BARRIER, 0)
     same_arrays(engines[0].evolve(rules, roots, steps, quotient=quotient, max_states=cap), want, barrier)
+
+
+def test_one_state_of_many_matches_reserves_the_pairs_it_has():
+    """14,280 matches of one state: 102 million possible pairs, of which 3.4 million share an edge."""
+    eng = Engine(0)
+    star = [[1, k] for k in range(2, 122)]
+    res = eng.evolve([([[0, 1], [0, 2]], [[1, 2]])], [star], 1, quotient=False)
+    assert len(res.events) == 120 * 119
+    assert len(res.branchial) == 14280 * (4 * 118 + 1) // 2   # (each shares an edge with 4 * 118 + 1 others)
+    assert eng.device_bytes() < 200 << 20
+    eng.close()
