@@ -1249,10 +1249,12 @@ struct Engine::Impl {
         std::vector<uint32_t> ids;
         uint64_t max_label = 0;
         // dedup table slots per evolution: enough for its small levels without a rehash (32,768 for a
-        // single one, cleared in 2 us), a million slots over a batch, at least 256 each
+        // single one, cleared in 2 us), a million slots over a run, at least 256 each. A session's
+        // tables stay until it is idle, so its evolutions count together however they come: 5,000
+        // small requests admitted one by one held 2 GB of tables at 32,768 slots each
         // (256 each under a device-memory ceiling, which they could otherwise reach before the run does)
         uint64_t table_slots = budget.limit ? 256 : 32768;
-        while (table_slots > 256 && table_slots * specs.size() > (1u << 20)) table_slots >>= 1;
+        while (table_slots > 256 && table_slots * (evo0 + specs.size()) > (1u << 20)) table_slots >>= 1;
         for (size_t i = 0; i < specs.size(); ++i) {
             const EvolutionSpec& spec = *specs[i];
             Packed& q = pk[i];

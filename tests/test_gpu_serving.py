@@ -80,3 +80,23 @@ def test_memory_budget_binds_and_results_equal_alone():
             assert_same(norm_gpu(rec.result), norm_gpu(alone), f"request {rec.rid}")
     finally:
         eng.close()
+
+
+def test_tables_of_a_long_session_stay_small():
+    """2,000 small requests, one admission each, in a session that is never idle: 393 KB of dedup table
+    each would be 786 MB."""
+    from hypergraphrewritingengine_b200 import Engine
+    eng = Engine(0)
+    eng.serve_reset()
+    ev = W.Evolution(rules=[([[0, 1]], [[0, 1], [1, 2]])], roots=[[[1, 2]]], steps=2, max_states=64)
+    jobs, keep = eng.make_jobs([ev])
+    for _ in range(2000):
+        eng.serve_admit(jobs[0])
+    assert eng.device_bytes() < 256 << 20
+    eng.serve_step()
+    eng.serve_step()
+    done = eng.serve_take_finished()
+    assert len(done) == 2000
+    alone = norm_gpu(eng.serve_collect(done[0]))
+    assert_same(norm_gpu(eng.serve_collect(done[-1])), alone, "last request")
+    eng.close()
