@@ -1,4 +1,6 @@
 """Evolutions of states past 256 edges (positions of more than a byte) against the oracle."""
+import time
+
 import numpy as np
 import pytest
 
@@ -55,3 +57,26 @@ def test_positions_past_a_byte(eng, name, forwarding):
     for s in sorted({0, 1, 7, len(res.state_hash) // 2, len(res.state_hash) - 1}):
         if s < len(res.state_hash):
             assert pyoracle.wl_hash(_edges(res, s)) == int(res.state_hash[s]), (name, s)
+
+
+@pytest.mark.parametrize("rule", [([[0, 1], [0, 2]], [[1, 2]]), ([[0, 1]], [[0, 1], [0, 2]])])
+def test_hub_vertex_join_index(eng, rule):
+    """A vertex in every edge: its list in the join index ascends (matches in canonical order, as without
+    the index), and building it for every unit of work does not cost the square of its degree."""
+    n = 150 if len(rule[0]) == 2 else 1500
+    star = [[1, k] for k in range(2, n)] + [[1, 1], [2, 1], [1, 2]]
+    out, ms = [], []
+    for index in (0, 1):
+        eng.set_option(api.OPT_JOIN_INDEX, index)
+        best = 1e9
+        for _ in range(3):
+            t = time.perf_counter()
+            res = eng.evolve([rule], [star], 1, quotient=False, max_states=3000)
+            best = min(best, time.perf_counter() - t)
+        out.append(res)
+        ms.append(1e3 * best)
+    eng.set_option(api.OPT_JOIN_INDEX, 1)
+    assert np.array_equal(out[0].events, out[1].events)
+    assert np.array_equal(out[0].event_cons, out[1].event_cons)
+    assert np.array_equal(out[0].state_hash, out[1].state_hash)
+    assert ms[1] < 3 * ms[0] + 2, ms
