@@ -202,7 +202,8 @@ __host__ __device__ Layout make_layout(uint32_t NE, uint32_t NOCC, const RuleMax
     NOCC = std::max<uint32_t>(NOCC, 1);
     L.NE = NE;
     L.NOCC = NOCC;
-    L.CNE = NE + rm.rhs;   // (at most 4,095 edges: see warp_shape)
+    L.CNE = NE + rm.rhs;
+    while ((1u << L.QS) < rm.arity) ++L.QS;
     L.CNOCC = NOCC + rm.rhs_total;
     L.NV = NV ? std::min(std::max<uint32_t>(NV, 1), NOCC) : NOCC;
     L.V = L.NV + rm.fresh;
@@ -332,6 +333,10 @@ __host__ __device__ Layout make_layout(uint32_t NE, uint32_t NOCC, const RuleMax
     L.bytes = align_up(off, 16);
     return L;
 }
+
+// Whether a warp can hold a state of this layout: its shared memory, and its edges in the bits that an
+// occurrence leaves them (65,536 unary ones, 32,768 of arity 2, 4,096 of arity 9 to 16).
+bool layout_fits(const Layout& L) { return L.bytes <= kMaxDynSmem && L.CNE <= (65536u >> L.QS); }
 
 #include "fused_levels.cuh"
 
@@ -1146,7 +1151,7 @@ struct Engine::Impl {
 
     template <class K>
     LaunchShape warp_shape(K kernel, const Layout& L, uint64_t items) {
-        if (L.bytes > kMaxDynSmem || L.CNE > 4095)
+        if (!layout_fits(L))
             throw std::runtime_error("hgx: a state exceeds the per-warp shared-memory capacity (" +
                                      std::to_string(L.bytes) + " bytes needed)");
         uint32_t wpb = static_cast<uint32_t>(std::min<size_t>(8, std::max<size_t>(1, (96 * 1024) / L.bytes)));
@@ -3135,7 +3140,7 @@ extern "C" HGX_API hgx_status hgx_hash_states_noalloc(
         RuleMax rm;
         rm.arity = kMaxArity;
         const Layout L = make_layout(max_edges, max_occ, rm, LayoutKind::Warp);
-        if (L.bytes > kMaxDynSmem || L.CNE > 4095)
+        if (!layout_fits(L))
             return noalloc_fail(HGX_ERR_CAPACITY,
                                 "hgx_hash_states_noalloc: states of this size exceed shared memory");
         int dev = 0;

@@ -1084,7 +1084,8 @@ __device__ bool parent_connected(const Layout& L, char* sm, const Parent& pa) {
 // FNV fold, in ascending order, of one vertex's neighbour words when they do not fit the buffer: the
 // warp finds the smallest word above the last one and how often it occurs, until all are folded.
 __device__ uint64_t fold_oversize(const uint8_t* car, const uint16_t* cvo, const uint16_t* vloc,
-                                  const uint16_t* o, uint32_t dv, uint32_t left, const uint64_t* cur, uint64_t h) {
+                                  const uint16_t* o, uint32_t qs, uint32_t dv, uint32_t left, const uint64_t* cur,
+                                  uint64_t h) {
     const uint32_t lane = lane_id();
     uint64_t last = 0;
     bool any = false;
@@ -1092,7 +1093,7 @@ __device__ uint64_t fold_oversize(const uint8_t* car, const uint16_t* cvo, const
         uint64_t m = ~0ull;
         uint32_t c = 0;
         for (uint32_t j = lane; j < dv; j += 32) {
-            const uint32_t e = o[j] >> 4, q = o[j] & 15u, a = car[e], vo = cvo[e];
+            const uint32_t e = o[j] >> qs, q = o[j] & ((1u << qs) - 1u), a = car[e], vo = cvo[e];
             for (uint32_t k = 0; k < a; ++k) {
                 if (k == q) continue;
                 const uint64_t x = fnv(cur[vloc[vo + k]], k);
@@ -1144,7 +1145,8 @@ __device__ uint64_t warp_wl(const Layout& L, char* sm, uint32_t ne, uint32_t V, 
     uint64_t* cur = smp<uint64_t>(sm, L.o_cur);
     uint64_t* nxt = smp<uint64_t>(sm, L.o_nxt);
     uint64_t* buf = smp<uint64_t>(sm, L.o_buf);
-    uint16_t* occ = smp<uint16_t>(sm, L.o_occ);
+    uint16_t* occ = smp<uint16_t>(sm, L.o_occ);   // an occurrence: edge << qs | position
+    const uint32_t qs = L.QS, qm = (1u << qs) - 1u;
     uint32_t* ooff = smp<uint32_t>(sm, L.o_ooff);
     uint32_t* deg = smp<uint32_t>(sm, L.o_deg);
     uint32_t* nn = smp<uint32_t>(sm, L.o_nn);
@@ -1207,7 +1209,7 @@ __device__ uint64_t warp_wl(const Layout& L, char* sm, uint32_t ne, uint32_t V, 
         const uint32_t a = car[e], vo = cvo[e];
         for (uint32_t q = 0; q < a; ++q) {
             const uint32_t slot = atomicAdd(&comp[vloc[vo + q]], 1u);
-            occ[slot] = static_cast<uint16_t>((e << 4) | q);
+            occ[slot] = static_cast<uint16_t>((e << qs) | q);
         }
     }
     __syncwarp();
@@ -1247,7 +1249,7 @@ __device__ uint64_t warp_wl(const Layout& L, char* sm, uint32_t ne, uint32_t V, 
                     o[j] = k;
                 }
             uint64_t* kb = buf + base;
-            for (uint32_t j = 0; j < n; ++j) kb[j] = (static_cast<uint64_t>(car[o[j] >> 4]) << 8) | (o[j] & 15u);
+            for (uint32_t j = 0; j < n; ++j) kb[j] = (static_cast<uint64_t>(car[o[j] >> qs]) << 8) | (o[j] & qm);
             isort64(kb, n);
             uint64_t h = fnv(kFnvOffset, static_cast<uint64_t>(dv));
             for (uint32_t j = 0; j < n; ++j) {
@@ -1271,7 +1273,7 @@ __device__ uint64_t warp_wl(const Layout& L, char* sm, uint32_t ne, uint32_t V, 
             for (uint32_t a = 1; a <= static_cast<uint32_t>(kMaxArity); ++a)
                 for (uint32_t q = 0; q < a; ++q) {
                     uint32_t c = 0;
-                    for (uint32_t j = lane; j < n; j += 32) c += car[o[j] >> 4] == a && (o[j] & 15u) == q ? 1u : 0u;
+                    for (uint32_t j = lane; j < n; j += 32) c += car[o[j] >> qs] == a && (o[j] & qm) == q ? 1u : 0u;
                     c = warp_sum32(c);
                     for (uint32_t j = 0; j < c; ++j) h = fnv(fnv(h, a), q);
                 }
@@ -1290,7 +1292,7 @@ __device__ uint64_t warp_wl(const Layout& L, char* sm, uint32_t ne, uint32_t V, 
                 const uint16_t* o = occ + ooff[v];
                 uint32_t m = 0;
                 for (uint32_t j = 0, dv = deg[v]; j < dv; ++j) {
-                    const uint32_t e = o[j] >> 4, q = o[j] & 15u, a = car[e], vo = cvo[e];
+                    const uint32_t e = o[j] >> qs, q = o[j] & qm, a = car[e], vo = cvo[e];
                     for (uint32_t k = 0; k < a; ++k)
                         if (k != q) kb[m++] = fnv(cur[vloc[vo + k]], k);
                 }
@@ -1298,7 +1300,7 @@ __device__ uint64_t warp_wl(const Layout& L, char* sm, uint32_t ne, uint32_t V, 
             const uint64_t h = fold_any(kb, n, n_max, mine ? cur[v] : 0ull);
             if (mine && deg[v]) nxt[v] = h;
         }, [&](uint32_t v, uint32_t n) {
-            const uint64_t h = fold_oversize(car, cvo, vloc, occ + ooff[v], deg[v], n, cur, cur[v]);
+            const uint64_t h = fold_oversize(car, cvo, vloc, occ + ooff[v], qs, deg[v], n, cur, cur[v]);
             if (lane == 0) nxt[v] = h;
             __syncwarp();
         });

@@ -134,6 +134,7 @@ struct LevelArgs {
 struct Layout {
     uint32_t NE, NOCC, CNE, CNOCC, V, W;
     uint32_t LH;        // left-hand edges of the longest rule (match list stride)
+    uint32_t QS;        // bits of a position within an edge (warp WL: an occurrence is 16 bits)
     uint32_t BUF;       // warp WL: neighbour words in shared memory
     uint32_t NV;        // distinct vertices a staged state may have (V = NV + fresh variables)
     uint32_t o_cur, o_nxt, o_buf;                                   // u64

@@ -80,3 +80,17 @@ def test_hub_vertex_join_index(eng, rule):
     assert np.array_equal(out[0].event_cons, out[1].event_cons)
     assert np.array_equal(out[0].state_hash, out[1].state_hash)
     assert ms[1] < 3 * ms[0] + 2, ms
+
+
+def test_states_past_4096_edges(eng):
+    """Unary edges of one vertex, 3,560 at the start and 15 more a step: 16-bit occurrences in the warp
+    hash leave the edge all bits that the arity does not need."""
+    steps = 38
+    res = eng.evolve([([[0]], [[0]] * 16)], [[[1]] * 3560], steps, quotient=True)
+    sizes = [3560 + 15 * d for d in range(steps + 1)]
+    assert sizes[-1] > 4096 + 16
+    assert [int(h) for h in res.state_hash] == [pyoracle.wl_hash([[1]] * n) for n in sizes]
+    assert len(res.events) == sum(sizes[:-1])
+    assert len(res.branchial) == 0
+    for d in (0, 35, 37, steps):
+        assert np.diff(res.state_edge_off)[d] == sizes[d]
