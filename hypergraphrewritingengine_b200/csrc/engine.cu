@@ -183,8 +183,9 @@ constexpr uint32_t kLaneLevel = 1u << 20;
 // shorter than the per-range work streaming adds).
 constexpr uint64_t kStreamMinBytes = 64ull << 20;
 
-// Matches listed at a time by the warp path, and neighbour words of its WL rounds in shared memory.
-constexpr uint32_t kListMax = 32, kWlBuf = 640;
+// Matches listed at a time by the warp path (kListLong at most where a list starts at the parent's first
+// match), and neighbour words of its WL rounds in shared memory.
+constexpr uint32_t kListMax = 32, kListLong = 256, kWlBuf = 640;
 
 enum class LayoutKind { Count, Lane, Warp, Seg };
 
@@ -194,7 +195,8 @@ enum class LayoutKind { Count, Lane, Warp, Seg };
 // warp layout's per-vertex WL arrays and the vertex hash table are sized by it.
 __host__ __device__ Layout make_layout(uint32_t NE, uint32_t NOCC, const RuleMax& rm, LayoutKind kind,
                                        bool fwd = false, uint32_t mcap = kLaneJoinCap,
-                                       bool index = false, uint32_t NV = 0, uint32_t seg = 32) {
+                                       bool index = false, uint32_t NV = 0, uint32_t seg = 32,
+                                       uint32_t list = kListMax) {
     const bool wl = kind == LayoutKind::Warp;
     const bool lane = kind == LayoutKind::Lane || kind == LayoutKind::Seg;
     Layout L{};
@@ -228,7 +230,7 @@ __host__ __device__ Layout make_layout(uint32_t NE, uint32_t NOCC, const RuleMax
     L.o_mdepth = take(2 * kMaxPatternEdges, 2);
     L.LH = rm.lhs;
     if (wl) {
-        L.o_mpos = take(2 * rm.lhs * kListMax, 2);
+        L.o_mpos = take(2 * rm.lhs * list, 2);
         L.o_ppk = take(4 * std::min<uint32_t>(NE, +kSegEMax), 4);
         L.o_sprod = take(4 * kMaxPatternEdges, 4);
     }
@@ -2434,8 +2436,24 @@ struct Engine::Impl {
             const uint32_t mne = std::max<uint32_t>(fmax_ne, 1), mno = std::max<uint32_t>(fmax_nocc, 1);
             const Layout Ll = make_layout(std::min<uint32_t>(mne, kLaneEMax), mno, rm, LayoutKind::Lane, fwd,
                                           fmax_cnt, false, fmax_nv);
-            const Layout Lw = make_layout(mne, mno, rm, LayoutKind::Warp, fwd, kLaneJoinCap,
-                                          opt.join_index != 0, fmax_nv);
+            // Where a slice's matches can only be found by enumerating the parent's from the first one on
+            // (rules of more than four left-hand edges, forwarded states, large states without counts per
+            // 32 first edges): slices of about sqrt(children), so that enumerating and building stay in
+            // step, shorter where the launch would have less than four units an SM (twelve for the last
+            // kind, whose lanes walk in parallel). Against slices of 32 or less, time in this kernel: 91
+            // thousand events of forwarded 70-edge states 16.4 -> 5.3 ms, 23 thousand of a rule of five
+            // left-hand edges on 100 edges 92 -> 26 ms, 3,913 of three left-hand edges on 240 edges under
+            // a memory ceiling 12.1 -> 10.9 ms a call.
+            const bool joined_whole = fwd || rm.lhs > kLaneJoinLhs;
+            const bool listed_whole = joined_whole || (mne > uint32_t(kLaneEMax) && (!A.chunks || mne > 32 * kChunks));
+            auto long_slice = [&](uint64_t events) {
+                uint32_t s = 1;
+                while (s < kListLong && uint64_t(s) * kNumSMs * (joined_whole ? 4 : 12) < events) s <<= 1;
+                return s;
+            };
+            const uint32_t list = listed_whole ? std::max(long_slice(n_ev), kListMax) : +kListMax;
+            const Layout Lw = make_layout(mne, mno, rm, LayoutKind::Warp, fwd, kLaneJoinCap, opt.join_index != 0, fmax_nv,
+                                          32, list);
             // matches by lane walks; the warp join where it is asked for (rules of more than four
             // left-hand edges take it by themselves)
             const bool walk = opt.lane_join != 1;
@@ -2472,6 +2490,7 @@ struct Engine::Impl {
             auto expand = [&](uint32_t n_work, uint64_t n_children) {
                 // (a share of the children takes the warp path; one child is 20-100 us of a warp)
                 A.wslice = std::min<uint32_t>(slice_for(n_children / 4), kListMax);
+                A.lslice = std::min(std::max(long_slice(n_children), A.wslice), list);
                 A.f_begin = 0;
                 A.f_end = n_work;
                 HGX_CUDA_CHECK(cudaMemsetAsync(work.p + 1, 0, 2 * sizeof(uint32_t), st));

@@ -1595,8 +1595,8 @@ __device__ void enumerate_matches(const DevPtrs& P, const Layout& L, char* sm, c
     while (j < f.nd) fwd_emit(L, sm, R, dpos2 + j++ * kFwdMaxLhs, on_match);
 }
 
-// State positions (pattern order, L.LH apart) of the staged state's matches [lo, hi), at most
-// kListMax of them, into the layout's list; rn: the matches the count pass found. The join's
+// State positions (pattern order, L.LH apart) of the staged state's matches [lo, hi), as many as the
+// layout's list holds, into the layout's list; rn: the matches the count pass found. The join's
 // structures may be overwritten once this returns (they share their bytes with the WL arrays).
 // False (and an error flag) when the join finds another number of matches.
 __device__ bool list_matches(const DevPtrs& P, const Layout& L, char* sm, const DevRule& R, const Parent& pa,
@@ -1874,6 +1874,7 @@ __global__ void __launch_bounds__(256, 4) k_count(DevPtrs P, LevelArgs A, Layout
         // lane-per-child eligibility: few enough vertices and a bounded neighbour count
         bool lane_ok = pa.nvp <= A.lane_vmax && pa.ne <= kLaneEMax && pa.ne > 0;
         bool seg_ok = pa.nvp <= static_cast<uint32_t>(kLaneVMax) && pa.ne <= kLaneEMax && pa.ne > 0;
+        bool whole = false;   // matches that a slice can only find from the first one on
         uint32_t pnn_max = 0;
         if (lane_ok) {
             const uint8_t* pear = smp<uint8_t>(sm, L.o_pear);
@@ -1899,6 +1900,8 @@ __global__ void __launch_bounds__(256, 4) k_count(DevPtrs P, LevelArgs A, Layout
                 if (part && R.n_lhs > kLaneJoinLhs) continue;   // counted whole by part 0
                 const Fwd fw = fwd_prepare(P, A, L, sm, R, ev, pa, sid, true);
                 fwd_on = fw.on;
+                whole = whole || fw.on || R.n_lhs > kLaneJoinLhs ||
+                        (pa.ne > kLaneEMax && !(A.chunks && chunked(pa.ne)));
                 if (fw.on) cnt = fwd_count(P, L, sm, R, pa, fw);
                 else if (R.n_lhs <= kLaneJoinLhs)
                     cnt = lane_join_count(L, sm, R, pa, vm,
@@ -1913,7 +1916,7 @@ __global__ void __launch_bounds__(256, 4) k_count(DevPtrs P, LevelArgs A, Layout
             }
             __syncwarp();
         }
-        if (lane == 0 && part == 0) A.fmode[f] = (lane_ok ? 1 : 0) | (fwd_on ? 2 : 0) | (seg_ok ? 4 : 0);
+        if (lane == 0 && part == 0) A.fmode[f] = (lane_ok ? 1 : 0) | (fwd_on ? 2 : 0) | (seg_ok ? 4 : 0) | (whole ? 8 : 0);
     }
 }
 
@@ -1985,12 +1988,22 @@ __device__ __forceinline__ uint32_t children_of(const LevelArgs& A, uint32_t f) 
     return A.item_ev[(f + 1) * A.rules_stride] - A.item_ev[f * A.rules_stride];
 }
 
+// Most children of frontier state f in one work unit of the warp-per-child kernel.
+__device__ __forceinline__ uint32_t slice_of(const LevelArgs& A, uint32_t f) {
+    if (!(A.fmode[f] & 8u)) return A.wslice;
+    const uint32_t c = children_of(A, f);
+    uint32_t s = 4;
+    while (uint64_t(s) * s < c) s <<= 1;
+    return min(max(s, A.wslice), A.lslice);
+}
+
 // Slice counts of the work indices [f_begin, f_begin + n) for the warp-per-child kernel.
 __global__ void k_slice_counts(LevelArgs A, uint32_t n, uint32_t* cnt) {
     for (uint32_t w = blockIdx.x * blockDim.x + threadIdx.x; w < n; w += gridDim.x * blockDim.x) {
         const uint32_t f = frontier_at(A, A.f_begin + w);
         const uint32_t c = children_of(A, f);
-        cnt[w] = (A.fmode[f] & A.path) ? 0u : (c + A.wslice - 1) / A.wslice;
+        const uint32_t s = slice_of(A, f);
+        cnt[w] = (A.fmode[f] & A.path) ? 0u : (c + s - 1) / s;
     }
 }
 
@@ -2029,8 +2042,9 @@ __global__ void __launch_bounds__(256, 3) k_expand(DevPtrs P, LevelArgs A, Layou
                 if (A.soff[m] <= u) a = m; else b = m;
             }
             f = frontier_at(A, A.f_begin + a);
-            c_lo = (u - A.soff[a]) * A.wslice;
-            c_hi = c_lo + A.wslice;
+            const uint32_t s = slice_of(A, f);
+            c_lo = (u - A.soff[a]) * s;
+            c_hi = c_lo + s;
         }
         const uint8_t fm = A.fmode[f];
         if (((fm & A.path) != 0) != kLane) continue;

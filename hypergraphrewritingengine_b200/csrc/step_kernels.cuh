@@ -101,16 +101,18 @@ struct LevelArgs {
     const uint32_t* frng;
     uint32_t n_frng;
     // warp-per-child kernel: exclusive scan over the n_sw work indices of their parents' slice
-    // counts (soff[n_sw] = total); a slice is a run of wslice consecutive children
+    // counts (soff[n_sw] = total); a slice is a run of slice_of consecutive children
     const uint32_t* soff;
     uint32_t n_sw;
     uint8_t* fmode;             // [F] bit 0: within the lane path's limits; bit 1: forwarding;
-                                // bit 2: within the segment path's
+                                // bit 2: within the segment path's; bit 3: matches are enumerated
+                                // from the first one for every slice
     uint32_t fwd_mode;          // 0 off, 1 every eligible state, 2 states with >= 48 edges
     uint32_t ev_keys;           // event signature keys (0 = no event canonicalisation)
     uint32_t lane_vmax;         // largest child (vertices) of this level the lane path takes
     uint32_t path;              // the level's small-state kernel as its fmode bit: 1 lane, 4 segment
     uint32_t slice, wslice;     // segment and warp-per-child kernels: most children of a work unit
+    uint32_t lslice;            // ... of a warp-per-child unit whose parent has fmode bit 3 (slice_of)
     uint32_t* work;             // work-queue counters
     // select / assign
     uint32_t* flag_new;         // [n_events]

@@ -94,3 +94,50 @@ def test_states_past_4096_edges(eng):
     assert len(res.branchial) == 0
     for d in (0, 35, 37, steps):
         assert np.diff(res.state_edge_off)[d] == sizes[d]
+
+
+def _paths(edges, k):
+    """Positions of every path of k edges, in canonical (lexicographic) order."""
+    out = {}
+    for i, (a, b) in enumerate(edges):
+        out.setdefault(a, []).append((i, b))
+    found = []
+
+    def walk(v, taken):
+        if len(taken) == k:
+            found.append(list(taken))
+            return
+        for i, b in out.get(v, ()):
+            if i not in taken:
+                walk(b, taken + [i])
+
+    for i, (a, b) in enumerate(edges):
+        walk(b, [i])
+    return found
+
+
+@pytest.mark.parametrize("n,vertices,seed", [(48, 9, 1), (100, 25, 2)])
+def test_long_slices_of_a_long_rule(eng, n, vertices, seed):
+    """More than 20,000 matches of a rule of five left-hand edges: slices longer than the usual list."""
+    edges = np.random.default_rng(seed).integers(1, vertices + 1, (n, 2)).tolist()
+    want = _paths(edges, 5)
+    assert len(want) > 20000
+    rule = ([[k, k + 1] for k in range(5)], [[0, 5], [5, 6]])
+    eng.set_option(api.OPT_RECORD_BRANCHIAL, 0)
+    res = eng.evolve([rule], [edges], 1, quotient=True)
+    eng.set_option(api.OPT_RECORD_BRANCHIAL, 1)
+    assert np.array_equal(res.event_cons.reshape(-1, 5), np.array(want))
+
+
+def test_long_slices_of_forwarded_states(eng):
+    """90,000 events of 70-edge states, forwarded and joined again: the same arrays."""
+    edges = np.random.default_rng(5).integers(1, 31, (70, 2)).tolist()
+    rule = ([[0, 1], [1, 2], [2, 3]], [[0, 3], [3, 4]])
+    out = []
+    for forwarding in (0, 1):
+        eng.set_option(api.OPT_FORWARDING, forwarding)
+        out.append(eng.evolve([rule], [edges], 2, quotient=True))
+    eng.set_option(api.OPT_FORWARDING, 0)
+    assert len(out[0].events) > 80000
+    for name in ("state_hash", "events", "event_cons", "causal", "branchial"):
+        assert np.array_equal(getattr(out[0], name), getattr(out[1], name)), name
