@@ -203,9 +203,13 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_levels(DevPtrs P, FusedArg
                     uint32_t cnt = 0;
                     if (r < ev.rule_count) {
                         load_rule(sm, L, &P.rules[ev.rule_begin + r]);
-                        if (Rr.n_lhs <= kLaneJoinLhs) cnt = lane_join_count(L, sm, Rr, pa, vm);
-                        else warp_join(L, sm, Rr, pa, Rr.sched, -1, [&](uint32_t) { ++cnt; }, 0xFFFFFFFFu,
-                                       SkipCounter{&cnt, 0xFFFFFFFFu});
+                        if (Rr.n_lhs <= kLaneJoinLhs) {
+                            cnt = lane_join_count(L, sm, Rr, pa, vm, nullptr, 0, 1, kFusedEvents);
+                        } else {
+                            warp_join(L, sm, Rr, pa, Rr.sched, -1, [&](uint32_t) { ++cnt; }, kFusedJoin + 1,
+                                      SkipCounter{&cnt, kFusedJoin});
+                            if (cnt > kFusedJoin) cnt = kFusedEvents + 1;   // leave the level
+                        }
                     }
                     if (lane == 0) {
                         const uint32_t t = f * R + r;

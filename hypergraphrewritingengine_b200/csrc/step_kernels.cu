@@ -923,11 +923,12 @@ __device__ uint32_t index_walk(const Layout& L, const char* csm, const DevRule& 
 __device__ __forceinline__ bool chunked(uint32_t ne) { return ne > kLaneEMax && ne <= 32 * kChunks; }
 
 // Matches of (state, rule) by lane walks over every first edge, warp total. A state of at most 16
-// (8) edges gives each first edge 2 (4) lanes, which split the second position's candidates.
+// (8) edges gives each first edge 2 (4) lanes, which split the second position's candidates. A state of
+// more than 64 edges is not counted on once its matches pass `limit`.
 __device__ uint32_t lane_join_count(const Layout& L, const char* sm, const DevRule& R,
                                     const Parent& pa, const unsigned long long* vm,
                                     uint32_t* chunks = nullptr, uint32_t part = 0,
-                                    uint32_t n_parts = 1) {
+                                    uint32_t n_parts = 1, uint32_t limit = 0xFFFFFFFFu) {
     uint32_t c = 0;
     const uint32_t lane = lane_id();
     if (chunks && chunked(pa.ne)) {
@@ -948,6 +949,7 @@ __device__ uint32_t lane_join_count(const Layout& L, const char* sm, const DevRu
         return warp_sum32(c);
     }
     for (uint32_t b = 0; b < pa.ne; b += 32) {
+        if (b >= kLaneEMax && limit != 0xFFFFFFFFu && warp_sum32(c) > limit) break;
         if (b + lane >= pa.ne) continue;
         if (pa.ne <= kLaneEMax) c += lane_walk(L, sm, R, pa, b + lane, vm, [](uint32_t) {});
         else c += index_walk(L, sm, R, pa, b + lane, [](unsigned long long) {});

@@ -58,6 +58,10 @@ SINGLE.update({
     "edges-97-roots": (GROW, [_chain(97), _chain(40), _chain(97)], 1, True, 0),
     "no-match": ([([[0, 1, 2]], [[0, 1]])], [_chain(3)], 3, True, 0),
     "long-lhs": ([([[0, 1], [1, 2], [2, 3], [3, 4], [4, 5]], [[0, 5], [5, 6]])], [_chain(12)], 3, True, 0),
+    # counting stops: enumerated matches of one state, and those of a state past 64 edges
+    "long-lhs-1944": ([([[0, 1], [1, 2], [2, 3], [3, 4], [4, 5]], [[0, 5]])],
+                      [[[i, i + 1] for i in range(1, 13) for _ in range(3)]], 1, True, 0),
+    "star-19460": ([([[0, 1], [0, 2]], [[1, 2]])], [[[1, i] for i in range(2, 142)]], 1, True, 0),
     "20-levels": ([([[0, 1]], [[1, 0]])], [_chain(5)], 20, True, 0),    # more levels than one launch takes
 })
 
