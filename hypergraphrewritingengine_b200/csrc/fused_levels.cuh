@@ -148,9 +148,10 @@ __device__ void fused_scan(uint32_t* a, uint32_t n, uint32_t* sh) {
 __device__ uint32_t fused_pairs(const DevPtrs& P, uint32_t a, uint32_t end, uint32_t in, uint2* out) {
     const unsigned long long ma = P.ev_bmask[a];
     const bool exact = P.st_ne[in] <= 63;
+    const uint32_t na = P.rules[P.ev_rule[a]].n_lhs, ca = P.ev_coff[a];
     uint32_t n = 0;
     for (uint32_t c = a + 1; c < end && P.ev_in[c] == in; ++c) {
-        if ((ma & P.ev_bmask[c]) == 0ull || !(exact || share_edge(P, a, c))) continue;
+        if ((ma & P.ev_bmask[c]) == 0ull || !(exact || share_edge(P, na, P.ev_cons + ca, c))) continue;
         if (out) out[n] = make_uint2(a, c);
         ++n;
     }

@@ -1962,14 +1962,13 @@ __device__ __forceinline__ unsigned long long branch_mask(uint32_t n, uint32_t p
     return m;
 }
 
-// Whether two events consumed a common edge, by edge ids.
-__device__ bool share_edge(const DevPtrs& P, uint32_t a, uint32_t c) {
-    const uint32_t na = P.rules[P.ev_rule[a]].n_lhs, ca = P.ev_coff[a];
+// Whether an event that consumed the na edges `ids` shares one with event c.
+__device__ __forceinline__ bool share_edge(const DevPtrs& P, uint32_t na, const uint32_t* ids, uint32_t c) {
     const uint32_t nc = P.rules[P.ev_rule[c]].n_lhs, cc = P.ev_coff[c];
     bool share = false;
     for (uint32_t k = 0; k < nc && !share; ++k) {
         const uint32_t x = P.ev_cons[cc + k];
-        for (uint32_t m = 0; m < na; ++m) share |= P.ev_cons[ca + m] == x;
+        for (uint32_t m = 0; m < na; ++m) share |= ids[m] == x;
     }
     return share;
 }
@@ -3215,7 +3214,9 @@ __global__ void __launch_bounds__(256, 4) k_materialize(DevPtrs P, LevelArgs A, 
 // Parents of more than 63 edges: thread per event, walking the state's later events until the input
 // state changes. A pair's masks are tested first; only pairs whose masks meet are compared by edge
 // ids (5.1 ms with the ids of every pair, 3.3 with the masks, over 129 evolutions of 65-256-edge
-// states). One warp per state instead, as below, took 37 ms there: few states with thousands of events.
+// states). The event's own ids are read once: where most masks meet, reading them for every pair took
+// 62 against 54 ms (23 thousand events of five left-hand edges). One warp per state, as in k_bpairs, took
+// 37 ms over those 129 evolutions: few states with thousands of events.
 template <bool kEmit>
 __global__ void k_bpairs_walk(DevPtrs P, LevelArgs A) {
     const uint32_t end = A.ev_base + A.n_events;
@@ -3224,10 +3225,13 @@ __global__ void k_bpairs_walk(DevPtrs P, LevelArgs A) {
         if (P.st_ne[in] <= 63) continue;   // k_bpairs'
         uint32_t cnt = 0;
         const unsigned long long ma = P.ev_kept[a] ? P.ev_bmask[a] : 0ull;
+        const uint32_t na = P.rules[P.ev_rule[a]].n_lhs, ca = P.ev_coff[a];
+        uint32_t ids[kMaxPatternEdges];
+        for (uint32_t k = 0; k < na; ++k) ids[k] = P.ev_cons[ca + k];
         uint32_t out = kEmit ? A.boff[t] : 0u;
         if (ma)
             for (uint32_t c = a + 1; c < end && P.ev_in[c] == in; ++c) {
-                if ((ma & P.ev_bmask[c]) == 0ull || !share_edge(P, a, c)) continue;
+                if ((ma & P.ev_bmask[c]) == 0ull || !share_edge(P, na, ids, c)) continue;
                 if (kEmit) reinterpret_cast<uint2*>(A.bpairs)[out++] = make_uint2(a, c);
                 ++cnt;
             }
