@@ -1160,11 +1160,11 @@ __device__ uint64_t warp_wl(const Layout& L, char* sm, uint32_t ne, uint32_t V, 
     info.nbr = 0;
     if (ne == 0) return kEmptyStateHash;
 
-    // degrees and neighbour counts; comp: occurrences by position, a byte each (one arity of 2..4)
+    // degrees and neighbour counts; comp: occurrences by position, a byte each (one arity of 1..4)
     for (uint32_t v = lane; v < V; v += 32) { deg[v] = 0; nn[v] = 0; comp[v] = 0; }
     __syncwarp();
     const uint32_t a0 = car[0];
-    bool uni = a0 >= 2 && a0 <= 4;
+    bool uni = a0 >= 1 && a0 <= 4;
     for (uint32_t e = lane; e < ne; e += 32) {
         const uint32_t a = car[e], vo = cvo[e];
         uni = uni && a == a0;
@@ -1194,14 +1194,15 @@ __device__ uint64_t warp_wl(const Layout& L, char* sm, uint32_t ne, uint32_t V, 
     info.nocc = run_o;
     info.nbr = run_nn;   // sum over edges of a(a-1): neighbour entries per refinement round
     if (nv == 0) return 0;   // only arity-0 edges: the reference core returns 0
-    const bool counted = uni && dmax < 256;
-    // initial colours of a single arity: the positions in order with their multiplicities
+    const bool counted = uni && (dmax < 256 || a0 == 1);
+    // initial colours of a single arity: the positions in order with their multiplicities (of unary
+    // edges, which have no neighbours, the cap leaves one occurrence)
     if (counted)
         for (uint32_t v = lane; v < V; v += 32) {
             const uint32_t c = comp[v];
             uint64_t h = fnv(kFnvOffset, static_cast<uint64_t>(deg[v]));
             for (uint32_t q = 0; q < a0; ++q)
-                for (uint32_t j = (c >> (8 * q)) & 0xFFu; j; --j) h = fnv(fnv(h, a0), q);
+                for (uint32_t j = a0 == 1 ? 1u : (c >> (8 * q)) & 0xFFu; j; --j) h = fnv(fnv(h, a0), q);
             cur[v] = h;
         }
     __syncwarp();

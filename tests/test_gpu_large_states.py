@@ -1,8 +1,10 @@
 """Evolutions of states past 256 edges (positions of more than a byte) against the oracle."""
+import ctypes
 import time
 
 import numpy as np
 import pytest
+import torch
 
 from hypergraphrewritingengine_b200 import Engine, api
 from oracle import pyoracle
@@ -141,3 +143,29 @@ def test_long_slices_of_forwarded_states(eng):
     assert len(out[0].events) > 80000
     for name in ("state_hash", "events", "event_cons", "causal", "branchial"):
         assert np.array_equal(getattr(out[0], name), getattr(out[1], name)), name
+
+
+def test_hashed_states_past_the_segment_limits_share_the_gpu():
+    """hgx_hash_states_noalloc: 64 states of 200 edges, a warp each at once, not one after another."""
+    import test_zz_no_alloc as Z
+    from hypergraphrewritingengine_b200 import load_library
+    states = [np.random.default_rng(k).integers(1, 120, (200, 2)).tolist() for k in range(64)]
+    ms = []
+    for n in (1, 64):
+        dev = torch.device("cuda", 0)
+        bufs = [torch.from_numpy(a.view(np.int32 if a.itemsize == 4 else np.int64)).to(dev)
+                for a in Z._records(states[:n])]
+        out = [torch.empty(n, dtype=torch.int64, device=dev), torch.empty(n, dtype=torch.int32, device=dev)]
+        p = [ctypes.c_void_p(t.data_ptr()) for t in bufs + out]
+        best = 1e9
+        for _ in range(20):
+            torch.cuda.synchronize()
+            t = time.perf_counter()
+            status = load_library().hgx_hash_states_noalloc(
+                *p[:4], n, 200, 400, p[4], p[5], ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+            torch.cuda.synchronize()
+            best = min(best, time.perf_counter() - t)
+            assert status == 0
+        assert [int(h) & (2 ** 64 - 1) for h in out[0].tolist()] == [pyoracle.wl_hash(s) for s in states[:n]]
+        ms.append(1e3 * best)
+    assert ms[1] < 4 * ms[0], ms
