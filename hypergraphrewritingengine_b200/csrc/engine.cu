@@ -939,7 +939,9 @@ struct Engine::Impl {
             HGX_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
             HGX_CUDA_CHECK(cudaFuncSetAttribute(k_levels, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                 static_cast<int>(kFusedSmemMax)));
-            if (coop && occupancy(reinterpret_cast<const void*>(k_levels), kFusedThreads, kFusedSmemMax) >= 1)
+            int bps = 0;   // (not through occupancy(), which answers 1 where nothing fits)
+            HGX_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_levels, kFusedThreads, kFusedSmemMax));
+            if (coop && bps >= 1)
                 fused_grid = std::min<uint32_t>(kNumSMs, static_cast<uint32_t>(sms));
             fused_state.ensure(1, 0, st);
             HGX_CUDA_CHECK(cudaMemsetAsync(fused_state.p, 0, sizeof(FusedState), st));
