@@ -3,7 +3,7 @@
 Per-stage timing (HGX_OPT_TIMING = 1) turns the launch off, so the same call runs on both paths;
 every result array must be equal, ids and order included. The cases sit at the edges of the
 launch's rule: levels just below and above its event limit, states around 63 / 64 edges (branchial
-masks, lane walk against warp join) and 96 (join index), several rules and roots, unary and mixed
+masks, lane walks against index walks and the join index), several rules and roots, unary and mixed
 arities, a deleting rule, caps out of and within reach, evolutions that stop in different levels of
 one batch, and levels run one per call by the serving steps.
 """
@@ -66,18 +66,31 @@ SINGLE.update({
 })
 
 
+# Cases with no level inside the launch, and those with some.
+LEFT = {"long-lhs-1944", "star-19460"}
+PARTLY = {"cap-full", "cap-near", "ternary-5", "wpp-7", "wpp-full-4"}
+
+
 @pytest.mark.parametrize("reduce,keys", [(False, 0), (True, 3)])
 @pytest.mark.parametrize("name", sorted(SINGLE))
 def test_single_evolutions(engines, name, reduce, keys):
     rules, roots, steps, quotient, cap = SINGLE[name]
-    out = []
+    out, launches = [], []
     for eng in engines:
         eng.set_option(api.OPT_TRANSITIVE_REDUCTION, reduce)
         eng.set_option(api.OPT_EVENT_SIGNATURE_KEYS, keys)
         out.append(eng.evolve(rules, roots, steps, quotient=quotient, max_states=cap))
+        launches.append(eng.stage_times()[1])
         eng.set_option(api.OPT_TRANSITIVE_REDUCTION, False)
         eng.set_option(api.OPT_EVENT_SIGNATURE_KEYS, 0)
     same_arrays(*out, name)
+    # that the launch did run: a level of the ordinary pipeline is at least ten launches
+    if name in LEFT:
+        assert launches[0] > launches[1], launches
+    elif name in PARTLY:
+        assert launches[0] < launches[1] - 20, launches
+    else:
+        assert launches[0] < 10, launches
 
 
 @pytest.mark.parametrize("n,cap", [(1, 50), (37, 200), (300, 4096)])
@@ -86,6 +99,8 @@ def test_batches(engines, n, cap):
            for i in range(n)]
     for i, (a, b) in enumerate(zip(*(eng.evolve_batch(evs) for eng in engines))):
         same_arrays(a, b, i)
+    if n < 300:   # (300 start with more events than a level of the launch takes)
+        assert engines[0].stage_times()[1] < engines[1].stage_times()[1]
 
 
 def test_record_options_and_serving_steps(engines):
@@ -222,3 +237,34 @@ def test_one_state_of_many_matches_reserves_the_pairs_it_has():
     assert len(res.branchial) == 14280 * (4 * 118 + 1) // 2   # (each shares an edge with 4 * 118 + 1 others)
     assert eng.device_bytes() < 200 << 20
     eng.close()
+
+
+def test_two_engines_on_two_threads():
+    """Two cooperative launches at a time, each on its own engine's stream: every result as alone."""
+    import threading
+    names = ["wpp-full-4", "ternary-5", "edges-97", "edge-multi-root-3", "long-lhs"]
+    both = Engine(0), Engine(0)
+
+    def call(eng, name):
+        rules, roots, steps, quotient, cap = SINGLE[name]
+        return eng.evolve(rules, roots, steps, quotient=quotient, max_states=cap)
+
+    alone = {name: call(both[0], name) for name in names}
+    failed = []
+
+    def work(k):
+        try:
+            for i in range(60):
+                name = names[(i + k * 2) % len(names)]
+                same_arrays(call(both[k], name), alone[name], (k, i, name))
+        except BaseException as e:   # (reported by the main thread)
+            failed.append(e)
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for e in both:
+        e.close()
+    assert not failed, failed
