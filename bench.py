@@ -598,7 +598,7 @@ def sharded_batch(eng, dist, world, rank, barrier, per_rank=1024):
 
 
 def join_index_ab(eng, reps=3):
-    """The join with and without its vertex / signature indices (states past 96 edges), on the
+    """The join with and without its vertex / signature indices (states past 64 edges), on the
     batched workload (C4) and on a batch of large-state evolutions (256 draws of the same
     generator with 65-256 initial edges, 2-4 steps, cap 4096): device time of the warp-per-child
     expand kernel (the large-state path) and wall time of the whole batch, best of `reps`."""

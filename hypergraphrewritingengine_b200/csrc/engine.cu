@@ -3032,10 +3032,9 @@ __global__ void k_noalloc_classes(DevPtrs P, DevEvo ev, const uint64_t* hash, ui
 // Every other state is marked in cls[i], and that there are any, for k_noalloc_hash. 3 KB of shared memory a warp
 // in place of 13 (whose neighbour buffer has to allow arity 16), and a quarter of the instructions:
 // 200,003 states of 4-40 edges 3.46 -> 0.83 ms.
-__global__ void __launch_bounds__(256, 4) k_noalloc_seg(DevPtrs P, DevEvo ev, uint32_t n, uint32_t max_edges,
-                                                       uint32_t max_occ, uint32_t* counters, uint64_t* hash,
-                                                       uint32_t* cls, uint32_t ne_cap, uint32_t listn,
-                                                       uint32_t bytes) {
+__global__ void __launch_bounds__(256, 4) k_noalloc_seg(DevPtrs P, DevEvo ev, uint32_t n, uint32_t max_occ,
+                                                       uint32_t* counters, uint64_t* hash, uint32_t* cls,
+                                                       uint32_t ne_cap, uint32_t listn, uint32_t bytes) {
     extern __shared__ __align__(16) char smem[];
     constexpr uint32_t full = 0xFFFFFFFFu, TS = 128;
     __shared__ SegTables tables;
@@ -3090,7 +3089,7 @@ __global__ void __launch_bounds__(256, 4) k_noalloc_seg(DevPtrs P, DevEvo ev, ui
             continue;
         }
         WlInfo info;
-        const uint64_t h = seg_wl<32>(ne, 32, A, false, scr, ne_cap, listn, tables, [&](uint32_t k) -> uint32_t {
+        const uint64_t h = seg_wl<32>(ne, A, false, scr, ne_cap, listn, tables, [&](uint32_t k) -> uint32_t {
             const uint8_t* s = slot + k * A;
             return s[0] | (uint32_t(s[1]) << 8) | (A == 3 ? uint32_t(s[2]) << 16 : 0u);
         }, info);
@@ -3219,7 +3218,7 @@ extern "C" HGX_API hgx_status hgx_hash_states_noalloc(
         const uint32_t listn = std::max<uint32_t>(2 * ne_cap, std::min<uint32_t>(6 * ne_cap, 2 * std::min<uint32_t>(max_occ, 3 * kSegEMax)));
         const uint32_t sb = align_up(align_up(seg_scratch_bytes(32, ne_cap, listn), 16) + 128 * 5 + 3 * kSegEMax, 16);
         const uint32_t sgrid = static_cast<uint32_t>(std::min<uint64_t>((n_states + 7) / 8, kNumSMs * 4));
-        k_noalloc_seg<<<sgrid, 256, sb * 8, st>>>(P, ev, n_states, max_edges, max_occ, counters, d_hash, d_class,
+        k_noalloc_seg<<<sgrid, 256, sb * 8, st>>>(P, ev, n_states, max_occ, counters, d_hash, d_class,
                                                   ne_cap, listn, sb);
         HGX_CUDA_CHECK(cudaGetLastError());
         k_noalloc_hash<<<grid, 32 * wpb, L.bytes * wpb, st>>>(P, ev, n_states, counters, d_hash, d_class, L);

@@ -124,10 +124,10 @@ struct StageTimes {
            branchial = 0, roots = 0, total = 0;
     uint64_t launches = 0;   // kernels this engine launched during the run
     uint64_t expand_launches = 0;
-    uint64_t walk_launches = 0;      // lane-kernel launches that used the lane-parallel walk
+    uint64_t walk_launches = 0;      // small-state expand launches that used the lane-parallel walk
     uint64_t result_streamed = 0;    // 1: the result was copied out range by range during the run
     uint64_t result_chunks = 0;      // its chunks
-    // lane-per-child expand kernel (k_expand<true>)
+    // small-state expand kernels (lane or segment per child)
     uint64_t expand_bytes = 0;       // per-stage algorithmic bytes
     uint64_t expand_hbm_bytes = 0;   // bytes the fused kernel must move to/from HBM
     uint64_t children = 0;           // children built and WL-hashed

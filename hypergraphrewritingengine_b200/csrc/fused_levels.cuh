@@ -419,7 +419,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_levels(DevPtrs P, FusedArg
                         }
                         __syncwarp();
                         WlInfo info;
-                        const uint64_t h = seg_wl<32>(keep + Rr.n_rhs, 32, ar, joined, sm + L.o_seg, L.SEGE, L.SEGN,
+                        const uint64_t h = seg_wl<32>(keep + Rr.n_rhs, ar, joined, sm + L.o_seg, L.SEGE, L.SEGN,
                                                       tables, [&](uint32_t j) -> uint32_t {
                             if (j >= keep) return sprod[j - keep];
                             uint32_t p = j;   // the j-th kept edge: past every removed position at or before it

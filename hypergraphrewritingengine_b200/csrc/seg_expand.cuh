@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(256, 3) k_expand_seg(DevPtrs P, LevelArgs A, L
                 const uint32_t* prod = reinterpret_cast<const uint32_t*>(slot + 8);
                 const unsigned long long rm = *reinterpret_cast<const unsigned long long*>(slot);
                 WlInfo x;
-                const uint64_t h = seg_wl<S>(valid ? nec : 0u, pa.nvp + R.n_fresh, ar, joined, scr, L.SEGE,
+                const uint64_t h = seg_wl<S>(valid ? nec : 0u, ar, joined, scr, L.SEGE,
                                              L.SEGN, tables, [&](uint32_t i) -> uint32_t {
                     if (i >= keep) return prod[i - keep];
                     uint32_t p = i;   // the i-th kept edge: past every removed position at or before it

@@ -122,12 +122,12 @@ __device__ __forceinline__ uint32_t seg_distinct(uint64_t c, uint32_t alive_seg,
     return __popc(__ballot_sync(0xFFFFFFFFu, lead) & segmask);
 }
 
-// edge(i): the state's edge i < ne as its vertices' local ids, position q in byte q. Per segment:
-// ne (0: no state), V, A, connected (known to be one component). Returns the segment's hash on all
+// edge(i): the state's edge i < ne as its vertices' local ids (below S), position q in byte q. Per
+// segment: ne (0: no state), A, connected (known to be one component). Returns the segment's hash on all
 // its lanes. scr: the segment's scratch (seg_scratch_bytes, 8-byte aligned); ne_cap, listn the
 // sizes it was made for.
 template <int S, class EdgeAt>
-__device__ __forceinline__ uint64_t seg_wl(uint32_t ne, uint32_t V, uint32_t A, bool connected, char* scr,
+__device__ __forceinline__ uint64_t seg_wl(uint32_t ne, uint32_t A, bool connected, char* scr,
                                            uint32_t ne_cap, uint32_t listn, const SegTables& T,
                                            EdgeAt&& edge, WlInfo& info) {
     constexpr uint32_t full = 0xFFFFFFFFu;

@@ -68,7 +68,9 @@ typedef enum hgx_option {
        hgx/compat.hpp keeps this on and selects the ids by edge_identity. */
     HGX_OPT_KEEP_STATE_EDGES = 5,
     /* 1 = record per-stage device times (CUDA events on the engine stream); 2 = time the expand
-       kernel launches only (two events per launch; the other stages read 0). */
+       kernel launches only (two events per launch; the other stages read 0). With 1 every level runs
+       the ordinary pipeline, the small ones too that otherwise share one launch: the stage times are
+       that pipeline's, not those of an untimed call. */
     HGX_OPT_TIMING = 6,
     /* 1 (default) = copy the result to host memory; 0 = keep it on the device and report the
        counts only (hgx_result_count works, hgx_result_copy returns empty arrays). */
@@ -267,8 +269,8 @@ HGX_API hgx_status hgx_engine_stage_times(hgx_engine* engine, double* out_ms, ui
    kernels). out[0..4], lane-per-child kernel: bytes by the per-stage figures (join + rewrite +
    WL + dedup counted as separate HBM streams), bytes the fused kernel itself must move to or
    from HBM, children hashed, WL refinement rounds, launches. out[5..8], warp-per-child kernel:
-   the same first four figures; out[9] its total device time in nanoseconds; out[10] lane-kernel
-   launches that ran the lane-parallel walk (out has 11 entries). */
+   the same first four figures; out[9] its total device time in nanoseconds; out[10] launches of
+   the small-state kernels (lane or segment) that ran the lane-parallel walk (out has 11 entries). */
 HGX_API hgx_status hgx_engine_expand_stats(hgx_engine* engine, uint64_t* out);
 
 /* The last evolve call's result: out[0] = 1 if it was streamed (copied to the host range by

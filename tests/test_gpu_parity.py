@@ -236,7 +236,7 @@ def test_level_split_matches_oracle(engine, split):
 
 @pytest.mark.parametrize("join", [1, 2])
 def test_lane_join_variants_match_oracle(engine, join):
-    """Both joins of the small-state expand kernel (the autotuner's choices) give the same result."""
+    """Both joins of the small-state expand kernel give the same result."""
     from hypergraphrewritingengine_b200 import api
     engine.set_option(api.OPT_LANE_JOIN, join)
     try:
@@ -253,7 +253,7 @@ def test_lane_join_variants_match_oracle(engine, join):
 
 
 def _large_state_cases():
-    """Evolutions whose states pass 64 edges (the join indices apply past 96): served-workload draws
+    """Evolutions whose states pass 64 edges (where the join indices apply): served-workload draws
     with large initial states (up to 256 edges, rules with repeated variables among them), a
     100-edge hub, and two disconnected LHS edges (candidates from the signature buckets)."""
     out = []
@@ -272,7 +272,7 @@ def _large_state_cases():
 
 @pytest.mark.parametrize("index", [1, 0])
 def test_join_index_modes_match_oracle(engine, index):
-    """The join with and without the vertex / signature indices (states past 96 edges) gives the
+    """The join with and without the vertex / signature indices (states past 64 edges) gives the
     oracle's result, alone and in a batch, with and without match forwarding."""
     from hypergraphrewritingengine_b200 import api
     evs = _large_state_cases()
