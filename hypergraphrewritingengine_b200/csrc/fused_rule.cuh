@@ -19,9 +19,10 @@ constexpr uint32_t kFusedEvents = 16384;    // most events of a level (a thread 
 constexpr uint32_t kFusedJoin = 512;
 constexpr uint32_t kFusedEdges = 255;       // largest state record a level may produce
 // Most branchial pairs to make room for ahead of a level. The launch has no count of them before it
-// writes them, only the bound c (c - 1) / 2 of every state with c matches: 8 MB at this limit, 1 GB for
-// one state of 16,384 matches, of which the ordinary level, which counts first, needs a few percent.
-constexpr uint64_t kFusedPairs = 1u << 20;
+// writes them, only the bound c (c - 1) / 2 of every state with c matches: 64 MB at this limit (one state
+// of 4,096 matches), 1 GB for one of 16,384, of which the ordinary level, which counts first, needs a few
+// percent. (At 8 MB a batch of 23 evolutions lost a level to the ordinary pipeline: 4.83 -> 5.04 ms.)
+constexpr uint64_t kFusedPairs = 1u << 23;
 constexpr uint64_t kIdLimit = 0xFFFFFFF0ull;   // 32-bit ids end here
 
 // Why a level was left to the ordinary pipeline.
