@@ -187,7 +187,7 @@ def max_over_ranks(dist, value: float, device: str = "cuda") -> float:
 
 
 def profile_traffic():
-    """dram bytes per lane-expand launch from the committed ncu summary, if present."""
+    """dram bytes of the mean small-state expand launch, from the committed ncu summary, if present."""
     p = os.path.join(ROOT, "profiles", "k_expand.c2-8step.txt")
     if not os.path.exists(p):
         return None
@@ -458,7 +458,7 @@ def main():
                 "copy": "each finished frontier range's share of the result copied to page-locked "
                         "host memory on a second stream while the later ranges compute "
                         "(HGX_OPT_STREAM_RESULT)"},
-        "roofline": {"bound": "hbm", "kernel": "k_expand_lanes2 (lane expand)", "achieved": achieved, "peak": peak,
+        "roofline": {"bound": "hbm", "kernel": "k_expand_seg and k_expand_lanes2 (small-state expand; mean launch)", "achieved": achieved, "peak": peak,
                      "unit": "GB/s", "frac": (achieved / peak) if achieved else None,
                      "traffic": traffic, "peak_kind": f"{peak_kind} (copy bandwidth)",
                      "algorithmic_bytes_per_launch": per_launch_bytes,

@@ -2377,7 +2377,9 @@ struct Engine::Impl {
         // rather than one per lane, but for the largest levels of small binary states, which fill
         // the lanes and keep them on like work (C2's last levels, lane against segment: 7.2 against
         // 8.6 ms; C3 2.3 against 1.4 ms, the 1,024 random evolutions 65 against 25 ms, C2's level 7
-        // -- 989,694 children -- the same)
+        // -- 989,694 children -- the same). The line comes from that one rule: no binary rule of 10-16
+        // vertices a child was measured at 2^20 children or more. `uniform` and R are the whole run's: one
+        // request of another kind in a session sends every level of it to the lane kernel.
         const bool seg = R == 1 && uniform && !fwd &&
                          !(rm.arity == 2 && fmax_nv + rm.fresh <= 16 && n_ev >= kLaneLevel);
         A.path = seg ? 4u : 1u;

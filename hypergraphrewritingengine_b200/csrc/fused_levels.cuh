@@ -16,7 +16,8 @@
 //   barrier 4
 //   output      thread per event: the class representative's id (then the next level's count)
 //
-// What bounds it is latency: dependent loads and barriers (1.5-2 us each), not bytes or issue slots.
+// What bounds it is latency: dependent loads, first fetches of instructions and barriers (1.5-2 us each),
+// not bytes or issue slots (5 % of them used; of 77 warps waiting per issue 61 stand at a barrier).
 // So every stage spreads over the whole grid (one event per thread, children dealt to warps in equal
 // runs whatever their parents), and children are hashed one per warp: a lane needs 30-50 us for its
 // child, a warp 3-5 us. That stops paying once the children outnumber the warps several times;

@@ -5,8 +5,9 @@
 // records live in a few hundred bytes of shared memory a state and in registers. Compared with one
 // state per lane (lane_wl.cuh) nothing is kept in local memory, the lanes of a warp run the same
 // step on equal work (a vertex's neighbour list in place of a whole state), and a state takes a
-// few microseconds instead of tens, so a launch of few states finishes early. Bound by issue slots
-// and shared-memory latency. Of the ways to sort a vertex's neighbour words, measured on states of
+// few microseconds instead of tens, so a launch of few states finishes early. Bound by
+// instruction fetch and issue slots (half of them used; stalls by count: no instruction, fixed latency,
+// shared memory). Of the ways to sort a vertex's neighbour words, measured on states of
 // 4-40 binary edges (200,003 of them) and on C2: insertion in shared memory 0.83 ms and 9.5 ms,
 // registers for every length 0.94 and 9.5 ms, registers up to 8 words and ranks above 0.83 and 8.6 ms.
 //
