@@ -139,6 +139,7 @@ enum ErrorBits : uint32_t {
     kErrBadRule = 1u << 3,
     kErrTrDepth = 1u << 4,       // transitive reduction past 64 levels
     kErrBarrier = 1u << 6,       // a grid barrier's wait ran out
+    kErrPairs = 1u << 7,         // a level's branchial pairs pass 32 bits
     kErrJoinCount = 1u << 5,     // a state's matches differ between the count and expand passes
 };
 

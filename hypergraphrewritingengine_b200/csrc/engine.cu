@@ -487,7 +487,7 @@ struct Engine::Impl {
     DVec<uint32_t> frontier, next_frontier, counts, item_ev, item_cons, item_prod, item_fresh;
     DVec<uint32_t> work, flag_new, scan_new, flag_rep, flag_front, new_state_event, level_max;
     DVec<uint32_t> bcount, boff, bpairs, scan_sums, sync_buf, root_ids;
-    DVec<unsigned long long> stats, totals;
+    DVec<unsigned long long> stats, totals, level_sums;
     DVec<uint8_t> fmode, fin;
     DVec<uint32_t> fin_cnt, evo_frange, fin_ids, map_s, map_e, frng, slice_off, seg_off, chunks;
     DVec<unsigned long long> evo_new, ev_anc, ev_sig, evo_sigs;
@@ -953,6 +953,7 @@ struct Engine::Impl {
         level_max.ensure(8, 0, st);
         sync_buf.ensure(16, 0, st);
         stats.ensure(8, 0, st);
+        level_sums.ensure(5, 0, st);
         reset();
     }
 
@@ -979,6 +980,7 @@ struct Engine::Impl {
         evo_causal.release(st);
         evo_states.release(st);
         stats.release(st);
+        level_sums.release(st);
         totals.release(st);
         fmode.release(st);
         fin.release(st);
@@ -1088,6 +1090,7 @@ struct Engine::Impl {
         P.evo_stopped = evo_stopped.p;
         P.err = err.p;
         P.stats = stats.p;
+        P.level_sums = level_sums.p;
         return P;
     }
 
@@ -2349,7 +2352,7 @@ struct Engine::Impl {
         const size_t w1 = 5 + 4 * nevo;
         const unsigned long long* hs = sync_host(std::max<size_t>(w1, (7 * nevo + 9 + 1) / 2));
         k_sync1_pack<<<grid_for(std::max<size_t>(nevo, 1), 256), 256, 0, st>>>(
-            item_ev.p, item_cons.p, item_prod.p, item_fresh.p, NI, level_max.p, evo_classes.p,
+            item_ev.p, item_cons.p, item_prod.p, item_fresh.p, NI, level_max.p, level_sums.p, evo_classes.p,
             evo_states.p, opt.event_keys ? evo_sigs.p : nullptr, evo_first_ev.p, evo_last_ev.p,
             static_cast<uint32_t>(nevo), d_sync);
         check_launch();
@@ -2735,7 +2738,7 @@ struct Engine::Impl {
             A.n_frontier = F_eff;
         }
         // ---- sync 2: new states, next frontier, branchial pairs, errors (behind the ranges)
-        k_sync2_pack<<<1, 32, 0, st>>>(flag_rep.p, flag_front.p, boff.p, ne2, err.p, evo_classes.p,
+        k_sync2_pack<<<1, 32, 0, st>>>(flag_rep.p, flag_front.p, boff.p, ne2, err.p, level_sums.p, evo_classes.p,
                                        evo_states.p, evo_stopped.p, ds2 + 7 * nevo);
         check_launch();
         sync_st();
@@ -2749,6 +2752,9 @@ struct Engine::Impl {
         const uint32_t* s2 = hs2 + 7 * nevo;
         if (s2[3] & kErrTrDepth)
             throw std::invalid_argument("transitive reduction supports evolutions of at most 64 levels");
+        // (pairs are laid out by 32-bit offsets within a level, and by 32-bit ids between several evolutions)
+        if ((s2[3] & kErrPairs) || (nevo > 1 && n_bpairs + s2[2] >= kIdLimit))
+            throw std::runtime_error("hgx: 32-bit id space exhausted (branchial pairs)");
         if (s2[3]) throw std::runtime_error("hgx: device error flags 0x" + std::to_string(s2[3]));
         const uint32_t n_new = s2[0], n_front = s2[1], n_b = s2[2];
         for (size_t e = 0; e < nevo; ++e) {

@@ -212,6 +212,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_levels(DevPtrs P, FusedArg
                                       SkipCounter{&cnt, kFusedJoin});
                             if (cnt > kFusedJoin) cnt = kFusedEvents + 1;   // leave the level
                         }
+                        cnt = min(cnt, kFusedEvents + 1);   // (the level's sum stays within 32 bits)
                     }
                     if (lane == 0) {
                         const uint32_t t = f * R + r;

@@ -1822,6 +1822,7 @@ __global__ void k_admit(DevPtrs P, AdmitArgs G) {
     if (G.fresh) {
         if (t == 0) *P.err = 0;
         if (t < 8) P.stats[t] = 0;
+        if (t < 5) P.level_sums[t] = 0;
     }
 }
 
@@ -1924,10 +1925,27 @@ __global__ void __launch_bounds__(256, 4) k_count(DevPtrs P, LevelArgs A, Layout
     }
 }
 
+// Adds n[0..K) to the level's totals, over the threads of a block (all of them call). True on one thread
+// when a total passes the 32-bit ids: the scans that lay a level out are 32 bits wide and would wrap.
+template <uint32_t K>
+__device__ bool add_level_sums(unsigned long long* totals, const unsigned long long* n) {
+    __shared__ unsigned long long sums[K];
+    if (threadIdx.x < K) sums[threadIdx.x] = 0;
+    __syncthreads();
+    for (uint32_t k = 0; k < K; ++k) {
+        const unsigned long long x = warp_sum64(n[k]);
+        if (lane_id() == 0 && x) atomicAdd(&sums[k], x);
+    }
+    __syncthreads();
+    const unsigned long long x = threadIdx.x < K ? sums[threadIdx.x] : 0ull;
+    return x && atomicAdd(&totals[threadIdx.x], x) + x >= kIdLimit;
+}
+
 // Per-item counts scaled by the rule's consumed / produced / fresh sizes, for the scans.
 __global__ void k_item_sizes(DevPtrs P, LevelArgs A) {
     const uint32_t n = A.n_frontier * A.rules_stride;
     uint32_t max_cnt = 0;   // largest match count of a (state, rule): sizes the staged match list
+    unsigned long long sums[4] = {};
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
         const uint32_t f = t / A.rules_stride, r = t % A.rules_stride;
         const uint32_t sid = A.frontier[f];
@@ -1940,12 +1958,17 @@ __global__ void k_item_sizes(DevPtrs P, LevelArgs A) {
             cons = c * R.n_lhs;
             prod = c * R.n_rhs;
             fresh = c * R.n_fresh;
+            sums[0] += c;
+            sums[1] += static_cast<unsigned long long>(c) * R.n_lhs;
+            sums[2] += static_cast<unsigned long long>(c) * R.n_rhs;
+            sums[3] += static_cast<unsigned long long>(c) * R.n_fresh;
         }
         A.item_ev[t] = c;
         A.item_cons[t] = cons;
         A.item_prod[t] = prod;
         A.item_fresh[t] = fresh;
     }
+    if (add_level_sums<4>(P.level_sums, sums)) atomicMax(&A.level_max[0], 1u);
     max_cnt = warp_max32(max_cnt);
     if (lane_id() == 0 && max_cnt) atomicMax(&A.level_max[4], max_cnt);
 }
@@ -2327,14 +2350,17 @@ __global__ void k_frontier_events(DevPtrs P, LevelArgs A, uint32_t* evo_last, ui
 // classes, states, event signatures (sigs may be null) and first | last event << 32.
 __global__ void k_sync1_pack(const uint32_t* item_ev, const uint32_t* item_cons,
                              const uint32_t* item_prod, const uint32_t* item_fresh, uint32_t ni,
-                             const uint32_t* level_max, const unsigned long long* classes,
+                             const uint32_t* level_max, unsigned long long* level_sums,
+                             const unsigned long long* classes,
                              const unsigned long long* states, const unsigned long long* sigs,
                              const uint32_t* first, const uint32_t* last, uint32_t nevo,
                              unsigned long long* out) {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     using u64 = unsigned long long;
     if (t == 0) {
-        out[0] = item_ev[ni] | (u64(item_cons[ni]) << 32);
+        // (a total past 32 bits: all ones, which no level fits)
+        out[0] = level_max[0] ? ~0ull : item_ev[ni] | (u64(item_cons[ni]) << 32);
+        for (uint32_t k = 0; k < 4; ++k) level_sums[k] = 0;
         out[1] = item_prod[ni] | (u64(item_fresh[ni]) << 32);
         out[2] = level_max[2] | (u64(level_max[3]) << 32);
         out[3] = level_max[4] | (u64(level_max[5]) << 32);
@@ -2355,6 +2381,7 @@ __global__ void k_sync1_pack(const uint32_t* item_ev, const uint32_t* item_cons,
 // round trips of their own.
 __global__ void k_sync2_pack(const uint32_t* flag_rep, const uint32_t* flag_front,
                              const uint32_t* boff, uint32_t ne2, const uint32_t* err,
+                             unsigned long long* level_sums,
                              const unsigned long long* classes, const unsigned long long* states,
                              const uint32_t* stopped, uint32_t* out) {
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -2367,6 +2394,7 @@ __global__ void k_sync2_pack(const uint32_t* flag_rep, const uint32_t* flag_fron
         out[6] = static_cast<uint32_t>(states[0]);
         out[7] = static_cast<uint32_t>(states[0] >> 32);
         out[8] = stopped[0];
+        level_sums[4] = 0;
     }
 }
 
@@ -3222,6 +3250,7 @@ __global__ void __launch_bounds__(256, 4) k_materialize(DevPtrs P, LevelArgs A, 
 template <bool kEmit>
 __global__ void k_bpairs_walk(DevPtrs P, LevelArgs A) {
     const uint32_t end = A.ev_base + A.n_events;
+    unsigned long long total = 0;
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < A.n_events; t += gridDim.x * blockDim.x) {
         const uint32_t a = A.ev_base + t, in = P.ev_in[a];
         if (P.st_ne[in] <= 63) continue;   // k_bpairs'
@@ -3238,7 +3267,9 @@ __global__ void k_bpairs_walk(DevPtrs P, LevelArgs A) {
                 ++cnt;
             }
         if (!kEmit) A.bcount[t] = cnt;
+        total += cnt;
     }
+    if (!kEmit && add_level_sums<1>(P.level_sums + 4, &total)) atomicOr(P.err, kErrPairs);
 }
 
 // Warp per input state (frontier position f, events [item_ev[f R], item_ev[(f+1) R]) of the level)
@@ -3249,6 +3280,7 @@ __global__ void k_bpairs(DevPtrs P, LevelArgs A) {
     const uint32_t lane = lane_id();
     const uint32_t warps = gridDim.x * (blockDim.x >> 5);
     const uint32_t R = A.rules_stride;
+    unsigned long long total = 0;
     for (uint32_t f = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); f < A.n_frontier; f += warps) {
         const uint32_t g0 = A.item_ev[f * R];
         const uint32_t g1 = min(A.item_ev[(f + 1) * R], A.n_events);
@@ -3276,8 +3308,10 @@ __global__ void k_bpairs(DevPtrs P, LevelArgs A) {
                 }
             }
             if (!kEmit && mine) A.bcount[g0 + i] = cnt;
+            total += cnt;
         }
     }
+    if (!kEmit && add_level_sums<1>(P.level_sums + 4, &total)) atomicOr(P.err, kErrPairs);
 }
 
 // ------------------------------------------------------------------------------------------

@@ -69,6 +69,9 @@ struct DevPtrs {
     // per event: the parent positions it consumed as a bit mask for the branchial test (branch_mask);
     // bit 63 alone: the event is not kept
     unsigned long long* ev_bmask;
+    // the level's totals in 64 bits: events, consumed entries, produced edges, fresh vertices, pairs
+    // (zero between levels)
+    unsigned long long* level_sums;
     // event canonicalisation: per event its signature; per evolution the distinct signatures
     unsigned long long* ev_sig;
     unsigned long long* evo_sigs;
@@ -122,7 +125,7 @@ struct LevelArgs {
     uint32_t state_base;
     uint32_t* new_state_event;  // [n_new] event of each new state
     uint32_t* next_frontier;
-    uint32_t* level_max;        // [2..3] max ne, nocc of the frontier;
+    uint32_t* level_max;        // [0] 1: a total passes 32 bits; [2..3] max ne, nocc of the frontier;
                                 // [4] largest match count of a (state, rule); [5] frontier
                                 // states for the warp path
     // branchial

@@ -169,3 +169,29 @@ def test_hashed_states_past_the_segment_limits_share_the_gpu():
         assert [int(h) & (2 ** 64 - 1) for h in out[0].tolist()] == [pyoracle.wl_hash(s) for s in states[:n]]
         ms.append(1e3 * best)
     assert ms[1] < 4 * ms[0], ms
+
+
+@pytest.mark.parametrize("spare", [0, 30])
+def test_pairs_of_a_level_past_32_bits(eng, spare):
+    """124,950 matches of one state that all hold its one loop: 7.8 billion branchial pairs, an error
+    before any is written (of a 52-edge state by the warp's count, of an 82-edge one by the walk)."""
+    star = [[1, 1]] + [[1, k] for k in range(2, 53)] + [[100 + 2 * k, 101 + 2 * k] for k in range(spare)]
+    rule = ([[0, 0], [0, 1], [0, 2], [0, 3]], [[1, 2]])
+    with pytest.raises(api.HgxError, match="branchial pairs") as err:
+        eng.evolve([rule], [star], 1, quotient=True)
+    assert err.value.status == api.HGX_ERR_CAPACITY
+    eng.set_option(api.OPT_RECORD_BRANCHIAL, 0)   # without them the level is an ordinary one
+    res = eng.evolve([rule], [star], 1, quotient=True)
+    eng.set_option(api.OPT_RECORD_BRANCHIAL, 1)
+    assert len(res.events) == 51 * 50 * 49
+    small = eng.evolve([rule], [star[:8]], 1, quotient=True)   # and the engine goes on
+    assert len(small.branchial) == 210 * 209 // 2
+
+
+def test_events_of_a_level_past_32_bits(eng):
+    """301 states of 14,295,960 matches each: more events than 32-bit ids, an error before any is built."""
+    roots = [[[r, 1000 + 63 * r + k] for k in range(63)] for r in range(301)]
+    with pytest.raises(api.HgxError, match="32-bit id space exhausted") as err:
+        eng.evolve([([[0, 1], [0, 2], [0, 3], [0, 4]], [[1, 2]])], roots, 1, quotient=True)
+    assert err.value.status == api.HGX_ERR_CAPACITY
+    assert len(eng.evolve([([[0, 1], [0, 2]], [[1, 2]])], [roots[0]], 1).events) == 63 * 62
