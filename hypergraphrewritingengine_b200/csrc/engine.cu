@@ -2713,6 +2713,9 @@ struct Engine::Impl {
         A.boff = boff.p;
         if (opt.branchial && ne2) {
             tic();
+            // (at most c (c - 1) / 2 a state; most levels cannot pass 32 bits and skip the sum's atomics,
+            // 40 us of a C2 evolution)
+            A.sum_pairs = uint64_t(ne2) * std::min<uint64_t>(uint64_t(fmax_cnt) * R, ne2) / 2 >= kIdLimit ? 1u : 0u;
             k_bpairs<false><<<grid_for(uint64_t(F_eff) * 32, 256), 256, 0, st>>>(ptrs(), A);
             check_launch();
             if (fmax_ne > 63) {

@@ -3269,7 +3269,7 @@ __global__ void k_bpairs_walk(DevPtrs P, LevelArgs A) {
         if (!kEmit) A.bcount[t] = cnt;
         total += cnt;
     }
-    if (!kEmit && add_level_sums<1>(P.level_sums + 4, &total)) atomicOr(P.err, kErrPairs);
+    if (!kEmit && A.sum_pairs && add_level_sums<1>(P.level_sums + 4, &total)) atomicOr(P.err, kErrPairs);
 }
 
 // Warp per input state (frontier position f, events [item_ev[f R], item_ev[(f+1) R]) of the level)
@@ -3311,7 +3311,7 @@ __global__ void k_bpairs(DevPtrs P, LevelArgs A) {
             total += cnt;
         }
     }
-    if (!kEmit && add_level_sums<1>(P.level_sums + 4, &total)) atomicOr(P.err, kErrPairs);
+    if (!kEmit && A.sum_pairs && add_level_sums<1>(P.level_sums + 4, &total)) atomicOr(P.err, kErrPairs);
 }
 
 // ------------------------------------------------------------------------------------------

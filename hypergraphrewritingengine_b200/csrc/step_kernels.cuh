@@ -129,6 +129,7 @@ struct LevelArgs {
                                 // [4] largest match count of a (state, rule); [5] frontier
                                 // states for the warp path
     // branchial
+    uint32_t sum_pairs;         // the level's pairs may pass 32 bits: sum them in 64
     uint32_t* bcount;           // [n_events] pairs (a, later b) per event a
     uint32_t* boff;             // [n_events+1] exclusive scan of bcount
     uint32_t* bpairs;           // output pairs (a, b)
